@@ -1,10 +1,10 @@
 // C-ABI implementation: context, scratch arena, launch sequence.
 //
 // One batch = columns x frequencies.  Launch sequence on the caller's stream:
-//   k_atmo      column pre-processing + output levels        (thread/column)
-//   k_gas       Rosenkranz-98 gas absorption                 (thread/layer-frequency)
-//   k_psd       size distributions                           (thread/layer-species)
-//   k_compact   list of hydrometeor-bearing layers           (one block)
+//   k_atmo      column pre-processing + output levels        (warp/column)
+//   k_gas       Rosenkranz-98 gas absorption                 (8 threads/layer-frequency)
+//   k_psd       size distributions                           (warp/layer-species)
+//   k_compact   list of hydrometeor-bearing layers           (warp/column)
 //   k_mie       Mie + species sums -> Legendre coefficients  (warp/layer-frequency, persistent)
 //   k_layer<N>  scatcnv + doubling -> layer R, T, S          (CTA/layer-frequency, persistent)
 //   k_adding<N> adding + radiance + TB                       (CTA/column-frequency, persistent)
@@ -238,7 +238,7 @@ struct Plan {
   size_t o_hgt_lev, o_temp_lev, o_temp, o_press, o_rho_vap, o_q_hum, o_vap, o_gtemp, o_outlev, o_kgas;
   size_t o_slot_st, o_slot_nb, o_bd, o_bdd, o_bnd, o_brho, o_bmass;
   size_t o_pres_idx, o_plist, o_counters, o_mkext, o_msalb, o_mback, o_mrefr, o_mnleg, o_mlegen, o_lay, o_laynd, o_status,
-      o_colst;
+      o_colst, o_colcnt;
   size_t o_species, o_addscr, o_mieslab, o_addstk;
   int mie_nslab;  // k_mie warps the slabs are sized for
   bool f32_coef;
@@ -307,6 +307,7 @@ Plan make_plan(const pamtra_b200_columns* c, int default_nummu, int sms, int mie
   p.o_laynd = take(items * 4);
   p.o_status = take(C * Fm * 4);
   p.o_colst = take(C * 4);
+  p.o_colcnt = take(C * 4);
   p.o_species = take(std::max<size_t>(nsp, 1) * sizeof(pamtra_b200_species));
   p.add_grid = (mask & 4) ? std::max(1, sms) : 0;
   p.o_addscr = take((size_t)p.add_grid * (10 - AddSmem<32>::NS) * RTCfg<32>::MAT * 8);
@@ -340,7 +341,7 @@ __global__ void k_gas_elem(const double* f, const double* T, const double* rv, c
                                   int32_t* st, int n) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
-  int s = gas_r98(f[i], T[i], rv[i], p[i], &k[i]);
+  int s = gas_r98<1>(f[i], T[i], rv[i], p[i], &k[i]);
   if (st) st[i] = s;
 }
 
@@ -863,7 +864,7 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   w.lay = (double*)(A + pl.o_lay); w.lay_stride = pl.lay_stride; w.lay_nd = (int*)(A + pl.o_laynd);
   w.lay32 = pl.tc_add ? 1 : 0;
   w.add_stk = pl.tc_add ? (float*)(A + pl.o_addstk) : nullptr;
-  w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst);
+  w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst); w.col_cnt = (int*)(A + pl.o_colcnt);
   w.add_scr = (double*)(A + pl.o_addscr);
   w.mie_slab = (double*)(A + pl.o_mieslab); w.mie_nslab = pl.mie_nslab;
   w.spin_limit = ctx->spin_limit;
@@ -902,19 +903,19 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
       launches++;
     }
   }
-  k_atmo<<<(unsigned)((C + 127) / 128), 128, 0, stream>>>(b, w); launches++;
+  k_atmo<<<(unsigned)((C + 3) / 4), 128, 0, stream>>>(b, w); launches++;
   const size_t ngas = C * Fm * Lm;
-  k_gas<<<(unsigned)((ngas + 255) / 256), 256, 0, stream>>>(b, w, st->lgas_extinction, st->gas_mod); launches++;
+  launch_gas(b, w, st->lgas_extinction, st->gas_mod, ngas, stream); launches++;
   mark(ctx, stream, STG_PREP);
   if (H > 0) {
     const size_t ns = C * Lm * H;
     if (cc.fs_d) k_fullspec<<<(unsigned)((ns + 127) / 128), 128, 0, stream>>>(b, w, *st);
-    else k_psd<<<(unsigned)((ns + 127) / 128), 128, 0, stream>>>(b, w, *st);
+    else k_psd<<<(unsigned)((ns + PSD_WARPS - 1) / PSD_WARPS), 32 * PSD_WARPS, 0, stream>>>(b, w, *st);
     launches++;
   } else {
     cudaMemsetAsync(w.slot_st, 0, 1, stream);
   }
-  k_compact<<<1, 1024, 0, stream>>>(b, w); launches++;
+  launches += launch_compact(b, w, stream);
   mark(ctx, stream, STG_PSD);
   const int sms = ctx->sm_count;
   if (H > 0) {
@@ -1442,7 +1443,7 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   w.m_legen = pl.f32_coef ? nullptr : (double*)(A + pl.o_mlegen);
   w.m_legen32 = pl.f32_coef ? (float*)(A + pl.o_mlegen) : nullptr;
   w.lay = (double*)(A + pl.o_lay); w.lay_stride = pl.lay_stride; w.lay_nd = (int*)(A + pl.o_laynd);
-  w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst);
+  w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst); w.col_cnt = (int*)(A + pl.o_colcnt);
   w.spin_limit = tc::MBAR_SPIN_LIMIT;
   w.mie_slab = (double*)(A + pl.o_mieslab); w.mie_nslab = pl.mie_nslab;
   w.gq_x = D.tables; w.gq_w = D.tables + gqn; w.gq_max = NOALLOC_GQ;
@@ -1455,9 +1456,9 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   const size_t ntb = (size_t)cc.noutlevels * 2 * cc.max_nummu * Fm * 2;
   k_fill_d<<<(unsigned)((ntb + 255) / 256), 256, 0, stream>>>(out->tb, -9999.0, ntb);
   k_atmo<<<1, 128, 0, stream>>>(b, w);
-  k_gas<<<(unsigned)((Fm * Lm + 255) / 256), 256, 0, stream>>>(b, w, st->lgas_extinction, st->gas_mod);
-  if (nh > 0) k_psd<<<(unsigned)((Lm * nh + 127) / 128), 128, 0, stream>>>(b, w, *st);
-  k_compact<<<1, 1024, 0, stream>>>(b, w);
+  launch_gas(b, w, st->lgas_extinction, st->gas_mod, Fm * Lm, stream);
+  if (nh > 0) k_psd<<<(unsigned)((Lm * nh + PSD_WARPS - 1) / PSD_WARPS), 32 * PSD_WARPS, 0, stream>>>(b, w, *st);
+  launch_compact(b, w, stream);
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   if (nh > 0) {

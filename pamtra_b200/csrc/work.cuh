@@ -57,6 +57,7 @@ struct Work {
   // compaction
   int* pres_idx;                       // [C][Lm]
   int* plist;                          // [pmax]
+  int* col_cnt;                        // [C] hydrometeor-bearing layers per column (k_present)
   int pmax;
   int* counters;                       // [16] 0: P, 1: mie work, 2-4: layer work, 5-7: adding work,
                                        // 8-9: n x n products of the FP64 layer kernel (uint64)
