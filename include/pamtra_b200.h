@@ -255,7 +255,9 @@ int32_t pamtra_b200_graph_destroy(pamtra_b200_graph* graph);
 int32_t pamtra_b200_set_wait_limit(pamtra_b200_ctx* ctx, uint32_t polls);
 
 /* n x n matrix products the FP64 doubling kernels (k_layer<N>) of the last
- * pamtra_b200_run on ctx issued, inverses by Gauss-Jordan counted as one:
+ * pamtra_b200_run on ctx issued, by the multiply-adds issued (a product with a
+ * symmetric result counts the share of it that is computed; a Gauss-Jordan
+ * inverse as one):
  * the executed counterpart of the algorithmic count of DOUBLING_INTEGRATION4
  * (src/radintg4.f90:174-309: six products and one inverse per doubling).
  * The split-precision kernels are not counted.  Waits for `stream`. */

@@ -944,8 +944,8 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   mark(ctx, stream, STG_MIE);
   double* ssp = out->scatter_matrix;
   if (mask & 1) {
-    int g = persistent_grid((const void*)k_layer<8>, RTCfg<8>::T, sizeof(LayerSmem<8>), sms, ctx->layer_cps);
-    if (H > 0) { k_layer<8><<<g, RTCfg<8>::T, sizeof(LayerSmem<8>), stream>>>(b, w, *st, ssp); launches++; }
+    int g = persistent_grid((const void*)k_layer<8>, LayerCfg<8>::T, sizeof(LayerSmem<8>), sms, ctx->layer_cps);
+    if (H > 0) { k_layer<8><<<g, LayerCfg<8>::T, sizeof(LayerSmem<8>), stream>>>(b, w, *st, ssp); launches++; }
     mark(ctx, stream, STG_LAYER);
     g = persistent_grid((const void*)k_adding<8>, RTCfg<8>::T, sizeof(AddSmem<8>), sms, ctx->adding_cps);
     if (one_inv) k_adding<8, true><<<g, RTCfg<8>::T, sizeof(AddSmem<8>), stream>>>(b, w, *st, *out);
@@ -962,8 +962,8 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
       const int g = (ctx->layer_cps > 0 ? std::min(ctx->layer_cps, 3) : 3) * sms;
       k_layer_tc<16><<<g, 128, smb, stream>>>(b, w, *st, ssp); launches++;
     } else if (H > 0) {
-      int g = persistent_grid((const void*)k_layer<16>, RTCfg<16>::T, sizeof(LayerSmem<16>), sms, ctx->layer_cps);
-      k_layer<16><<<g, RTCfg<16>::T, sizeof(LayerSmem<16>), stream>>>(b, w, *st, ssp); launches++;
+      int g = persistent_grid((const void*)k_layer<16>, LayerCfg<16>::T, sizeof(LayerSmem<16>), sms, ctx->layer_cps);
+      k_layer<16><<<g, LayerCfg<16>::T, sizeof(LayerSmem<16>), stream>>>(b, w, *st, ssp); launches++;
     }
     mark(ctx, stream, STG_LAYER);
     if (pl.tc_add) {
@@ -982,12 +982,12 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
     mark(ctx, stream, STG_ADDING);
   }
   if (mask & 4) {
-    int g = persistent_grid((const void*)k_layer<32>, RTCfg<32>::T, sizeof(LayerSmem<32>), sms, ctx->layer_cps);
+    int g = persistent_grid((const void*)k_layer<32>, LayerCfg<32>::T, sizeof(LayerSmem<32>), sms, ctx->layer_cps);
     if (H > 0 && split) {
       // one item per CTA, one CTA per SM (165 KB shared memory, 256 TMEM columns)
       k_layer_tc64<<<sms, 256, layer_tc64_smem(), stream>>>(b, w, *st, ssp); launches++;
     } else if (H > 0) {
-      k_layer<32><<<g, RTCfg<32>::T, sizeof(LayerSmem<32>), stream>>>(b, w, *st, ssp); launches++;
+      k_layer<32><<<g, LayerCfg<32>::T, sizeof(LayerSmem<32>), stream>>>(b, w, *st, ssp); launches++;
     }
     mark(ctx, stream, STG_LAYER);
     g = std::min(persistent_grid((const void*)k_adding<32>, RTCfg<32>::T, sizeof(AddSmem<32>), sms, ctx->adding_cps),
@@ -1467,11 +1467,11 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
     k_mie<MIE_GROUP><<<NOALLOC_MIE_SLABS / MIE_WARPS, 32 * MIE_WARPS, sm_mie, stream>>>(b, w, *st);
   }
   if (mask & 1) {
-    if (nh > 0) k_layer<8><<<sms, RTCfg<8>::T, sizeof(LayerSmem<8>), stream>>>(b, w, *st, out->scatter_matrix);
+    if (nh > 0) k_layer<8><<<sms, LayerCfg<8>::T, sizeof(LayerSmem<8>), stream>>>(b, w, *st, out->scatter_matrix);
     k_adding<8><<<sms, RTCfg<8>::T, sizeof(AddSmem<8>), stream>>>(b, w, *st, *out);
   }
   if (mask & 2) {
-    if (nh > 0) k_layer<16><<<sms, RTCfg<16>::T, sizeof(LayerSmem<16>), stream>>>(b, w, *st, out->scatter_matrix);
+    if (nh > 0) k_layer<16><<<sms, LayerCfg<16>::T, sizeof(LayerSmem<16>), stream>>>(b, w, *st, out->scatter_matrix);
     k_adding<16><<<sms, RTCfg<16>::T, sizeof(AddSmem<16>), stream>>>(b, w, *st, *out);
   }
   if (out->angles_deg) k_angles<<<1, 32, 0, stream>>>(out->angles_deg, w.lob_mu, cc.max_nummu);

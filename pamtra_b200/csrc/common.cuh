@@ -82,6 +82,12 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
+// sum over the four lanes of a quad (lanes 4g .. 4g + 3)
+__device__ __forceinline__ double quad_sum(double v) {
+  v += __shfl_xor_sync(0xffffffffu, v, 1);
+  return v + __shfl_xor_sync(0xffffffffu, v, 2);
+}
+
 // ------------------------------------------------------------------ team linear algebra
 // A "team" is one CTA working on n x n FP64 matrices (n = 16, 32, 64) held in
 // shared memory, column-major with leading dimension LD = n + 4 (LD = 4 mod
@@ -103,6 +109,29 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
                : "+d"(d[0]), "+d"(d[1])
                : "d"(a), "d"(b));
+}
+
+// An 8 x 8 accumulator tile (row block i, column block j) to and from a
+// column-major matrix.  A lane holds row g of columns 2q and 2q + 1; with
+// LD = 4 mod 16 the lanes of q and q + 2 meet in a bank when all lanes take
+// column 2q first, so q >= 2 takes 2q + 1 first: two wavefronts per access, the least
+// for 32 doubles, instead of four.
+template <int n>
+__device__ __forceinline__ void store_tile(double* C, int i, int j, const double (&c)[2]) {
+  constexpr int LD = Team<n>::LD;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, o = q >> 1;
+  double* p = C + (8 * j + 2 * q) * LD + 8 * i + g;
+  p[o * LD] = o ? c[1] : c[0];
+  p[(1 - o) * LD] = o ? c[0] : c[1];
+}
+template <int n>
+__device__ __forceinline__ void load_tile(const double* C, int i, int j, double (&c)[2]) {
+  constexpr int LD = Team<n>::LD;
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, o = q >> 1;
+  const double* p = C + (8 * j + 2 * q) * LD + 8 * i + g;
+  const double x = p[o * LD], y = p[(1 - o) * LD];
+  c[0] = o ? y : x;
+  c[1] = o ? x : y;
 }
 
 enum MMMode { MM_SET = 0, MM_ACC = 1, MM_IMINUS = 2, MM_IPLUS = 3 };
@@ -127,9 +156,13 @@ __device__ __forceinline__ void mm(const double* A, const double* B, double* C, 
 #pragma unroll
       for (int i = 0; i < 2; i++) {
         const int row = row0 + rt * 8 + g, col = col0 + ct * 8 + 2 * q + i;
-        c[rt][ct][i] = (MODE == MM_ACC) ? D[col * LD + row]
-                                        : ((MODE == MM_IMINUS || MODE == MM_IPLUS) ? (row == col ? 1.0 : 0.0) : 0.0);
+        c[rt][ct][i] = (MODE == MM_IMINUS || MODE == MM_IPLUS) ? (row == col ? 1.0 : 0.0) : 0.0;
       }
+  if (MODE == MM_ACC)
+#pragma unroll
+    for (int rt = 0; rt < 2; rt++)
+#pragma unroll
+      for (int ct = 0; ct < 2; ct++) load_tile<n>(D, (row0 >> 3) + rt, (col0 >> 3) + ct, c[rt][ct]);
   const double sgn = (MODE == MM_IMINUS) ? -1.0 : 1.0;
 #pragma unroll 4
   for (int kk = 0; kk < n; kk += 4) {
@@ -146,12 +179,7 @@ __device__ __forceinline__ void mm(const double* A, const double* B, double* C, 
 #pragma unroll
   for (int rt = 0; rt < 2; rt++)
 #pragma unroll
-    for (int ct = 0; ct < 2; ct++)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int row = row0 + rt * 8 + g, col = col0 + ct * 8 + 2 * q + i;
-        C[col * LD + row] = c[rt][ct][i];
-      }
+    for (int ct = 0; ct < 2; ct++) store_tile<n>(C, (row0 >> 3) + rt, (col0 >> 3) + ct, c[rt][ct]);
 }
 
 // Two products with the same left factor in one pass over K:
@@ -171,13 +199,11 @@ __device__ __forceinline__ void mm2(const double* A, const double* B1, double* C
 #pragma unroll
   for (int rt = 0; rt < 2; rt++)
 #pragma unroll
-    for (int ct = 0; ct < 2; ct++)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int row = row0 + rt * 8 + g, col = col0 + ct * 8 + 2 * q + i;
-        c[rt][ct][i] = (MODE1 == MM_ACC) ? D1[col * LD + row] : 0.0;
-        e[rt][ct][i] = (MODE2 == MM_ACC) ? D2[col * LD + row] : 0.0;
-      }
+    for (int ct = 0; ct < 2; ct++) {
+      c[rt][ct][0] = c[rt][ct][1] = e[rt][ct][0] = e[rt][ct][1] = 0.0;
+      if (MODE1 == MM_ACC) load_tile<n>(D1, (row0 >> 3) + rt, (col0 >> 3) + ct, c[rt][ct]);
+      if (MODE2 == MM_ACC) load_tile<n>(D2, (row0 >> 3) + rt, (col0 >> 3) + ct, e[rt][ct]);
+    }
 #pragma unroll 4
   for (int kk = 0; kk < n; kk += 4) {
     const double a0 = A[(kk + q) * LD + row0 + g];
@@ -198,14 +224,69 @@ __device__ __forceinline__ void mm2(const double* A, const double* B1, double* C
 #pragma unroll
   for (int rt = 0; rt < 2; rt++)
 #pragma unroll
-    for (int ct = 0; ct < 2; ct++)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int row = row0 + rt * 8 + g, col = col0 + ct * 8 + 2 * q + i;
-        C1[col * LD + row] = c[rt][ct][i];
-        C2[col * LD + row] = e[rt][ct][i];
-      }
+    for (int ct = 0; ct < 2; ct++) {
+      store_tile<n>(C1, (row0 >> 3) + rt, (col0 >> 3) + ct, c[rt][ct]);
+      store_tile<n>(C2, (row0 >> 3) + rt, (col0 >> 3) + ct, e[rt][ct]);
+    }
 }
+
+// ------------------------------------------------------------------ symmetric-matrix teams
+// A team of n / 8 warps works on symmetric n x n matrices (and one general
+// one, kept transposed): warp i owns the 8-row strip i of every result.  A
+// matrix is held column by column with leading dimension n, the 16-byte
+// chunks of a column (two rows) XOR-swizzled, so that the three access
+// patterns below take the least number of wavefronts:
+//   fragment: lane (g, q) reads rows 8u + 2q, + 1 of column 8j + g (16 bytes).
+//     As the left factor of a symmetric matrix that is M[8j+g][k], as the
+//     right factor M[k][8j+g], for the k pair 2q, 2q + 1 of block u: the two
+//     MMAs of the block take k = 8u + 2q and k = 8u + 2q + 1, so one 16-byte
+//     read serves both and a tile's accumulators (row g, columns 2q, 2q + 1) are
+//     themselves the left fragment of that tile: a result strip can be the
+//     left factor of the next product without leaving the registers;
+//   direct store of tile (i, j): column 8i + g, rows 8j + 2q, + 1 (16 bytes;
+//     the transposed tile, which for a symmetric matrix is its mirror image);
+//   mirror store: column 8j + 2q + e, row 8i + g (8 bytes).
+template <int n>
+struct SymTeam {
+  static constexpr int NB = n / 8, D = NB / 2, T = 32 * NB, MAT = n * n;
+  __device__ static __forceinline__ int swz(int col) { return (((col >> 1) & 3) << 1) ^ ((col & 1) << 2); }
+  // offset of element (row, col)
+  __device__ static __forceinline__ int at(int row, int col) {
+    return col * n + ((((row >> 1) ^ swz(col)) << 1) | (row & 1));
+  }
+  // offset of a lane's fragment of column block j, k block u
+  __device__ static __forceinline__ int frag(int j, int u) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    return (8 * j + g) * n + (((4 * u + q) ^ swz(g)) << 1);
+  }
+  __device__ static __forceinline__ double2 ld(const double* M, int j, int u) {
+    return *reinterpret_cast<const double2*>(M + frag(j, u));
+  }
+  __device__ static __forceinline__ void st(double* M, int i, int j, const double (&c)[2]) {
+    *reinterpret_cast<double2*>(M + frag(i, j)) = make_double2(c[0], c[1]);
+  }
+  // both halves of a symmetric result's tile (i, j); a diagonal tile keeps its upper triangle
+  __device__ static __forceinline__ void st_sym(double* M, int i, int j, const double (&c)[2]) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+    const int row = 8 * i + g, col = 8 * j + 2 * q;
+    if (i != j) {
+      st(M, i, j, c);
+#pragma unroll
+      for (int e = 0; e < 2; e++) M[at(row, col + e)] = c[e];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 2; e++)
+        if (row <= col + e) {
+          M[at(row, col + e)] = c[e];
+          M[at(col + e, row)] = c[e];
+        }
+    }
+  }
+  // The strip's share of a symmetric result: column blocks (i + d) mod NB for
+  // d < D, and d = D for half of the strips (which half differs between the two
+  // results of a pass, so every strip has NB + 1 tiles of a pair).
+  __device__ static __forceinline__ int blk(int i, int d) { return (i + d) & (NB - 1); }
+};
 
 // row `row` of M * x (k-ascending FMA chain)
 template <int n>
@@ -336,10 +417,9 @@ __device__ int ginv(double* A, InvScratch<n>& S) {
 // (Horner wins for the thin layers of the first doublings, where ||X|| is
 // tiny and G = I + X needs no product at all); otherwise Gauss-Jordan with
 // partial pivoting.  Returns the buffer holding the inverse (P or G); *sing
-// set on a zero pivot; *nprod (if given) grows by the n x n products the
-// inverse took (Gauss-Jordan counted as one: n^3 multiply-adds).
+// set on a zero pivot.
 template <int n>
-__device__ double* inv_iminus(double* P, double* G, InvScratch<n>& S, int* sing, int* nprod = nullptr) {
+__device__ double* inv_iminus(double* P, double* G, InvScratch<n>& S, int* sing) {
   constexpr int LD = Team<n>::LD, T = Team<n>::T;
   const int t = threadIdx.x;
   // infinity norm of X
@@ -378,7 +458,6 @@ __device__ double* inv_iminus(double* P, double* G, InvScratch<n>& S, int* sing,
       mm<n, MM_IPLUS, true>(P, G, G);  // G = I + X G
       team_sync();
     }
-    if (nprod) *nprod += kh;
     return G;
   }
   if (m >= 8) {
@@ -389,7 +468,6 @@ __device__ double* inv_iminus(double* P, double* G, InvScratch<n>& S, int* sing,
     }
     team_sync();
     if (ginv<n>(P, S)) *sing = 1;
-    if (nprod) *nprod += 1;
     return P;
   }
   // G = I + X
@@ -404,7 +482,6 @@ __device__ double* inv_iminus(double* P, double* G, InvScratch<n>& S, int* sing,
     mm<n, MM_ACC, true>(G, P, G, G);  // G = G + G P
     team_sync();
   }
-  if (nprod) *nprod += 2 * (m - 1);
   return G;
 }
 

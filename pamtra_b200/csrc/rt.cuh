@@ -48,23 +48,33 @@ __host__ __device__ __forceinline__ size_t lay_stride_n(int N) {
 }
 
 // ============================================================== layer kernel
+// With M = diag(mu_j w_j) the layer matrices of Mie spheres are symmetric in
+// the scaled form M^(1/2) R M^(-1/2) (reciprocity: the azimuth-mean phase
+// matrix of (I, Q) obeys P(mu1, mu2) = P(mu2, mu1)^T, and likewise for
+// (-mu1, mu2)), and doubling keeps them so.  k_layer carries R and T scaled.
 template <int N>
 struct LayerSmem {
-  static constexpr int n = RTCfg<N>::n, MAT = RTCfg<N>::MAT;
-  // matrices: R, T, G, W (and Y = R T as a fifth for N != 16).  For N = 16
-  // four matrices keep the block under 45.6 KB, so five CTAs fit per SM; the
-  // doubling then forms Y in G's buffer once G is consumed.  During scatcnv
-  // G (and W for N = 8) hold the coefficients, the last matrix the azimuth table.
-  static constexpr int NM = (N == 16) ? 4 : 5;
-  double m[NM][MAT];
-  double lin[2 * n], cst[2 * n];
-  double lin2[2 * n], cst2[2 * n];  // the other half of the doubled source buffers
-  double v[4][n], u[4][n];
+  static constexpr int n = 2 * N, LMAT = RTCfg<N>::MAT;
+  static constexpr int COEF = 3 * MAXNLEG;
+  // R, T, X and Y^T of the doubling (SymTeam layout); before it the set-up's R
+  // and T (column-major, leading dimension n + 4), coefficients and azimuth
+  // table; the elimination's I - X takes X and Y
+  static constexpr int M = (4 * SymTeam<n>::MAT > 2 * LMAT + COEF + 2 * KMAX) ? 4 * SymTeam<n>::MAT : 2 * LMAT + COEF + 2 * KMAX;
+  static_assert(LMAT <= 2 * SymTeam<n>::MAT, "the elimination's matrix fits X and Y");
+  alignas(16) double m[M];
+  alignas(16) double C[n], E[n];    // constant source C and e = o - f C / 2
+  alignas(16) double UC[n], UE[n];  // C + R C, e - R e
+  double o[n];                    // odd part of the linear source
+  double lin[2 * n], cst[2 * n];  // thin-layer sources of layer_setup
   double mu[N], wq[N], nrm[N];
+  double sc[n], is[n];            // sqrt(mu w) per row and its inverse
+  double fro[n / 8];              // sums of squares of the scaled R, per warp
   InvScratch<n> inv;
   int item, stat;
-  // set-up buffers (layer_setup): R, T, coefficients, azimuth table
-  __device__ __forceinline__ double* mat(int i) { return m[i < NM ? i : NM - 1]; }
+  // set-up buffers (layer_setup): 0 R, 1 T, 2 coefficients, 4 azimuth table
+  __device__ __forceinline__ double* mat(int k) {
+    return m + (k < 2 ? k * LMAT : 2 * LMAT + (k == 4 ? COEF : 0));
+  }
 };
 
 // Azimuth weights of scatcnv (src/scatcnv.f90:103-192 with SUM_LEGENDRE,
@@ -376,20 +386,62 @@ __device__ __forceinline__ void layer_store(const Work& w, int item, const doubl
   for (int e = t; e < 2 * n; e += T) out[2 * MAT + e] = lin[e];
 }
 
+// DOUBLING_INTEGRATION4, SYMMETRIC (src/radintg4.f90:174-309):
+//   R' = R + T G R T, T' = T G T with G = (I - R R)^-1,
+// as X = R R, Y = R T, W = T G, then R' = R + W Y and T' = W T; the source
+// chains use W u for T G u.  In the scaled form R, T, X, R' and T' are
+// symmetric, so three of the five products compute NB (NB + 1) / 2 of NB^2
+// tiles (10 of 16 for n = 32, 36 of 64 for n = 64).
+// The sources: the constant parts C+ and C- start equal and stay so; the
+// linear ones are S+- = (1 + a) C +- o, where the even part follows C (a grows by
+// f / 2 per step) and the odd part obeys
+//   o' = o + f C / 2 + W (I - R) e,  e = o - f C / 2,
+// so two mat-vec pairs carry the four chains of the reference:
+// C' = C + W (C + R C) and o'.  They take the fragments the passes hold anyway.
+// Three barriers per step:
+//   pass 1  X, Y^T = T R and the vectors C + R C, e - R e into shared memory;
+//   pass 2  the warp's strip of W, in registers: W = T + T X + ..., one product
+//           per term (W <- T + W X) with no barrier between them, since a strip
+//           of W is the left factor of its own next term; for thick layers
+//           W <- W + W X^(2^k) with X squared in place;
+//   pass 3  R', T' and the sources from the W strip (left factor, still in
+//           registers) with Y, T and those vectors, written after a barrier.
+// The trace of X = R R bounds its norm (X is positive semidefinite) and is
+// the sum of squares of R, known before X.
+// What bounds it: the FP64 tensor pipe, 77 % busy (66 % with five full products
+// in 16 x 16 tiles, 8-byte fragments and five barriers per step), then the
+// data path of shared memory (58 %).  1500 columns x 50 layers x 4 frequencies, NUMMU 16:
+// 30.6 -> 22.3 ms; 40 columns of mixed NUMMU: 27.3 -> 20.0 ms for the three kernels.
 template <int N>
-__global__ void __launch_bounds__(RTCfg<N>::T, (N == 16 ? 5 : 1)) k_layer(Batch b, Work w, pamtra_b200_settings st,
-                                                       double* __restrict__ ssp_scat) {
-  constexpr int n = RTCfg<N>::n, LD = RTCfg<N>::LD, MAT = RTCfg<N>::MAT, T = RTCfg<N>::T;
-  (void)LD;
-  (void)MAT;
+struct LayerCfg {
+  static constexpr int n = 2 * N, T = SymTeam<n>::T;
+  // resident CTAs the registers are bounded for.  N = 16: five (96 registers);
+  // six would fit shared memory but spill more and measure the same (22.2 ms).
+  static constexpr int CTAS = (N == 8) ? 8 : (N == 16) ? 5 : 1;
+};
+
+template <int N>
+__global__ void __launch_bounds__(LayerCfg<N>::T, LayerCfg<N>::CTAS) k_layer(Batch b, Work w, pamtra_b200_settings st,
+                                                                            double* __restrict__ ssp_scat) {
+  using TM = SymTeam<2 * N>;
+  constexpr int n = 2 * N, T = TM::T, NB = TM::NB, D = TM::D;
+  constexpr int LD = RTCfg<N>::LD, LMAT = RTCfg<N>::MAT;  // layout of layer_setup, the elimination and the layer records
   extern __shared__ double smem_raw[];
   LayerSmem<N>& S = *reinterpret_cast<LayerSmem<N>*>(smem_raw);
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, lane = t & 31, i = t >> 5;  // i: this warp's strip
+  const int g = lane >> 2, q = lane & 3;
+  const bool low = i < D;
   const int Fm = b.max_nfreq;
   const int P = min(w.counters[0], w.pmax);
   const int nitems = P * Fm;
   scat_weights_mark_ready<N>(w);
   if (t < N) { S.mu[t] = w.lob_mu[lob_off(N) + t]; S.wq[t] = w.lob_w[lob_off(N) + t]; }
+  if (t < n) {
+    const double v = sqrt(w.lob_mu[lob_off(N) + (t >> 1)] * w.lob_w[lob_off(N) + (t >> 1)]);
+    S.sc[t] = v;
+    S.is[t] = 1.0 / v;
+  }
+  double *const R = S.m, *const Tm = S.m + TM::MAT, *const X = S.m + 2 * TM::MAT, *const Y = S.m + 3 * TM::MAT;
   for (;;) {
     team_sync();
     if (t == 0) S.item = atomicAdd(&w.counters[2 + (N == 8 ? 0 : (N == 16 ? 1 : 2))], 1);
@@ -397,94 +449,288 @@ __global__ void __launch_bounds__(RTCfg<N>::T, (N == 16 ? 5 : 1)) k_layer(Batch 
     const int item = S.item;
     if (item >= nitems) break;
     LayerItem it;
-    if (!layer_setup<N>(b, w, st, ssp_scat, S, item, it)) continue;
+    if (!layer_setup<N, LayerSmem<N>, T>(b, w, st, ssp_scat, S, item, it)) continue;
     const int nd = it.nd, c = it.c, fi = it.fi;
     int status = it.status;
-    double linfac = it.linfac;
-    double* Rb = S.m[0];
-    double* Tb = S.m[1];
-    double* Gb = S.m[2];
-    double* Wb = S.m[3];
-    double* Yb = S.mat(4);  // = Gb's buffer role for N = 16 (see below)
-    constexpr bool FOUR = LayerSmem<N>::NM == 4;
-    // ---------------- DOUBLING_INTEGRATION4, SYMMETRIC (src/radintg4.f90:174-309)
-    // R' = R + T G R T and T' = T G T with G = (I - R R)^-1, as five products
-    // per step: W = T G, then R' = R + W (R T) and T' = W T; the source
-    // chains use W u for T G u.  R R and R T only read R and T, so they
-    // share the first phase.
-    constexpr int NV = (4 * n + T - 1) / T;
-    int nprod = 5 * nd;  // n x n products issued for this item (counted by thread 0)
-    // sources S+ / S- (linear and constant parts), double-buffered so that a
-    // step writes the new ones while other threads still read the old
-    double *lin = S.lin, *cst = S.cst, *lin_n = S.lin2, *cst_n = S.cst2;
-    for (int itd = 0; itd < nd; itd++) {
-      mm<n, MM_SET>(Rb, Rb, Gb);  // R+ R-
-      if (!FOUR) mm<n, MM_SET>(Rb, Tb, Yb);  // Y = R T
-      // v = [S- + f C-, C-, S+, C+]
-      for (int o = t; o < 4 * n; o += T) {
-        const int r = o % n, k = o / n;
-        double v;
-        if (k == 0) v = lin[n + r] + linfac * cst[n + r];
-        else if (k == 1) v = cst[n + r];
-        else if (k == 2) v = lin[r];
-        else v = cst[r];
-        S.v[k][r] = v;
-      }
-      team_sync();
-      {
-        int sg = 0;
-        double* gi = inv_iminus<n>(Gb, Wb, S.inv, &sg, &nprod);  // GAMMA = inv(I - R+ R-)
-        if (sg) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_PIVOT;
-        if (gi != Gb) { Wb = Gb; Gb = gi; }
-      }
-      // W = T G;  u = [S+ + R v0, C+ + R v1, v0 + R v2, C- + R v3]
-      mm<n, MM_SET>(Tb, Gb, Wb);
-      for (int o = t; o < 4 * n; o += T) {
-        const int r = o % n, k = o / n;
-        const double a = mv_row<n>(Rb, S.v[k], r);
-        double u;
-        if (k == 0) u = lin[r] + a;
-        else if (k == 1) u = cst[r] + a;
-        else if (k == 2) u = S.v[0][r] + a;
-        else u = cst[n + r] + a;
-        S.u[k][r] = u;
-      }
-      team_sync();
-      // new sources from W u, then R' = R + W Y and T' = W T (into the G
-      // buffer): nothing of this phase reads what it writes.  With four
-      // matrices Y = R T goes into G's buffer here (G is consumed), and T' is
-      // formed in place in T.
-      if (FOUR) mm<n, MM_SET>(Rb, Tb, Gb);
+    double f = it.linfac;
+    // scaled, symmetric R and T from the set-up's layout (through registers:
+    // the two layouts overlap); scaled sources
+    double fro = 0.0;
+    {
+      constexpr int E = (n * n + T - 1) / T;
+      double r[E], v[E];
 #pragma unroll
-      for (int s = 0; s < NV; s++) {
-        const int o = t + s * T;
-        if (o < 4 * n) {
-          const int r = o % n, k = o / n;
-          const double a = mv_row<n>(Wb, S.u[k], r);
-          if (k == 0) lin_n[r] = (lin[r] + a) + linfac * cst[r];
-          else if (k == 1) cst_n[r] = cst[r] + a;
-          else if (k == 2) lin_n[n + r] = lin[n + r] + a;
-          else cst_n[n + r] = cst[n + r] + a;
-        }
+      for (int k = 0; k < E; k++) {
+        const int e = t + k * T, col = e / n, row = e % n;
+        // exactly 1 on the diagonal: T is near the identity, whose rounding counts most
+        const double s1 = (row == col) ? 1.0 : S.sc[row] * S.is[col], s2 = (row == col) ? 1.0 : S.sc[col] * S.is[row];
+        const double *Rs = S.mat(0), *Ts = S.mat(1);
+        r[k] = 0.5 * (Rs[col * LD + row] * s1 + Rs[row * LD + col] * s2);
+        v[k] = 0.5 * (Ts[col * LD + row] * s1 + Ts[row * LD + col] * s2);
+        fro += r[k] * r[k];
       }
-      if (FOUR) {
-        team_sync();                           // Y complete
-        mm<n, MM_ACC>(Wb, Gb, Rb, Rb);         // R' = R + W Y
-        mm<n, MM_SET, true>(Wb, Tb, Tb);       // T' = W T (reads W and T, barrier, writes T)
-      } else {
-        mm<n, MM_ACC>(Wb, Yb, Rb, Rb);
-        mm<n, MM_SET>(Wb, Tb, Gb);
-        { double* tmp = Tb; Tb = Gb; Gb = tmp; }
-      }
-      { double* tmp = lin; lin = lin_n; lin_n = tmp; }
-      { double* tmp = cst; cst = cst_n; cst_n = tmp; }
-      linfac = 2.0 * linfac;
       team_sync();
+#pragma unroll
+      for (int k = 0; k < E; k++) {
+        const int e = t + k * T, col = e / n, row = e % n;
+        R[TM::at(row, col)] = r[k];
+        Tm[TM::at(row, col)] = v[k];
+      }
     }
-    layer_store<N>(w, item, Rb, Tb, lin);
+    fro = warp_sum(fro);
+    if (lane == 0) S.fro[i] = fro;
+    double even = 1.0;  // 1 + a
+    if (t < n) {  // INITIAL_SOURCE4 leaves all four sources equal
+      const double c0 = S.cst[t] * S.sc[t];
+      S.C[t] = c0;
+      S.o[t] = 0.0;
+      S.E[t] = -(0.5 * f) * c0;
+    }
+    int tiles = 0;  // 8 x 8 tiles of products issued for this item (counted by thread 0)
+    const int row = 8 * i + g;
+    for (int itd = 0; itd < nd; itd++) {
+      team_sync();
+      double nrm = 0.0;  // trace of X
+#pragma unroll
+      for (int k = 0; k < NB; k++) nrm += S.fro[k];
+      // ---- pass 1
+      {
+        double x[D + 1][2], y[NB][2], zc = 0.0, ze = 0.0;
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+#pragma unroll
+          for (int d = 0; d <= D; d++) x[d][e] = 0.0;
+#pragma unroll
+          for (int d = 0; d < NB; d++) y[d][e] = 0.0;
+        }
+#pragma unroll 2
+        for (int u = 0; u < NB; u++) {
+          const double2 a = TM::ld(R, i, u), at = TM::ld(Tm, i, u);
+#pragma unroll
+          for (int d = 0; d < NB; d++) {
+            const double2 bb = (d == 0) ? a : TM::ld(R, TM::blk(i, d), u);
+            if (d < D || (d == D && low)) {
+              dmma(x[d < D ? d : D], a.x, bb.x);
+              dmma(x[d < D ? d : D], a.y, bb.y);
+            }
+            dmma(y[d], at.x, bb.x);
+            dmma(y[d], at.y, bb.y);
+          }
+          const double2 vc = *reinterpret_cast<const double2*>(S.C + 8 * u + 2 * q);
+          const double2 ve = *reinterpret_cast<const double2*>(S.E + 8 * u + 2 * q);
+          zc = fma(a.y, vc.y, fma(a.x, vc.x, zc));
+          ze = fma(a.y, ve.y, fma(a.x, ve.x, ze));
+        }
+#pragma unroll
+        for (int d = 0; d < D; d++) TM::st_sym(X, i, TM::blk(i, d), x[d]);
+        if (low) TM::st_sym(X, i, TM::blk(i, D), x[D]);
+#pragma unroll
+        for (int d = 0; d < NB; d++) TM::st(Y, i, TM::blk(i, d), y[d]);
+        zc = quad_sum(zc);
+        ze = quad_sum(ze);
+        if (q == 0) S.UC[row] = S.C[row] + zc;
+        else if (q == 1) S.UE[row] = S.E[row] - ze;
+      }
+      team_sync();
+      // ---- pass 2
+      double W[NB][2];
+#pragma unroll
+      for (int u = 0; u < NB; u++) {
+        const double2 a = TM::ld(Tm, i, u);
+        W[u][0] = a.x;
+        W[u][1] = a.y;
+      }
+      // W <- (T or W) + W X
+      auto term = [&](bool add_t) {
+        double h[NB][2];
+#pragma unroll
+        for (int j = 0; j < NB; j++) {
+          h[j][0] = W[j][0];
+          h[j][1] = W[j][1];
+          if (add_t) {
+            const double2 a = TM::ld(Tm, i, j);
+            h[j][0] = a.x;
+            h[j][1] = a.y;
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < NB; u++)
+#pragma unroll
+          for (int j = 0; j < NB; j++) {
+            const double2 bb = TM::ld(X, j, u);
+            dmma(h[j], W[u][0], bb.x);
+            dmma(h[j], W[u][1], bb.y);
+          }
+#pragma unroll
+        for (int j = 0; j < NB; j++) { W[j][0] = h[j][0]; W[j][1] = h[j][1]; }
+      };
+      int kh = 0, m = 1;
+      if (nrm * nrm > 5.0e-17) {
+        if (nrm > 0.5) {
+          // the trace is a loose bound for thick layers: the row-sum norm of
+          // the unscaled X decides between the series and the elimination
+          if (t < n) {
+            double r = 0.0;
+            for (int j = 0; j < n; j++) r += fabs(X[TM::at(j, t)]) * S.sc[j];
+            r *= S.is[t];
+            const unsigned mask = (n >= 32) ? 0xffffffffu : ((1u << n) - 1u);
+#pragma unroll
+            for (int o = ((n >= 32) ? 16 : n / 2); o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(mask, r, o));
+            if ((t & 31) == 0) S.inv.cand_v[t >> 5] = r;
+          }
+          team_sync();
+          double rs = S.inv.cand_v[0];
+#pragma unroll
+          for (int k = 1; k < (n + 31) / 32; k++) rs = fmax(rs, S.inv.cand_v[k]);
+          nrm = fmin(nrm, rs);
+        }
+        // further terms: kh by Horner (remainder nrm^(kh + 2)) or m - 1 squarings (remainder nrm^(2^m))
+        for (double pw = nrm; pw > 5.0e-17 && m < 8; m++) pw = pw * pw;
+        for (double ph = nrm * nrm; ph > 5.0e-17 && kh < 2 * (m - 1); kh++) ph = ph * nrm;
+      }
+      if (m >= 8) {
+        // Gauss-Jordan on I - X in the column-major layout, over X and Y (Y waits in registers)
+        constexpr int E = n * n / T;
+        double x[E], y[E];
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+          const int e = t + k * T, col = e / n, r = e % n;
+          x[k] = ((r == col) ? 1.0 : 0.0) - X[TM::at(r, col)];
+          y[k] = Y[e];
+        }
+        team_sync();
+#pragma unroll
+        for (int k = 0; k < E; k++) { const int e = t + k * T; X[(e / n) * LD + e % n] = x[k]; }
+        team_sync();
+        if (ginv<n, T>(X, S.inv)) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_PIVOT;
+#pragma unroll
+        for (int k = 0; k < E; k++) {  // G - I
+          const int e = t + k * T, col = e / n, r = e % n;
+          x[k] = X[col * LD + r] - ((r == col) ? 1.0 : 0.0);
+        }
+        team_sync();
+#pragma unroll
+        for (int k = 0; k < E; k++) {
+          const int e = t + k * T;
+          X[TM::at(e % n, e / n)] = x[k];
+          Y[e] = y[k];
+        }
+        team_sync();
+        term(false);  // W = T + T (G - I)
+        tiles += 2 * NB * NB;
+      } else if (kh <= 7 * (m - 1) / 4) {
+        term(false);
+        for (int k = 0; k < kh; k++) term(true);
+        tiles += (kh + 1) * NB * NB;
+      } else {
+        // W = T (I + X)(I + X^2)(I + X^4)...
+        term(false);
+        for (int k = 1; k < m; k++) {
+          double x[D + 1][2];
+#pragma unroll
+          for (int d = 0; d <= D; d++) x[d][0] = x[d][1] = 0.0;
+          for (int u = 0; u < NB; u++) {
+            const double2 a = TM::ld(X, i, u);
+#pragma unroll
+            for (int d = 0; d <= D; d++)
+              if (d < D || low) {
+                const double2 bb = (d == 0) ? a : TM::ld(X, TM::blk(i, d), u);
+                dmma(x[d], a.x, bb.x);
+                dmma(x[d], a.y, bb.y);
+              }
+          }
+          team_sync();
+#pragma unroll
+          for (int d = 0; d < D; d++) TM::st_sym(X, i, TM::blk(i, d), x[d]);
+          if (low) TM::st_sym(X, i, TM::blk(i, D), x[D]);
+          team_sync();
+          term(false);
+        }
+        tiles += m * NB * NB + (m - 1) * (NB * (NB + 1) / 2);
+      }
+      // ---- pass 3
+      {
+        double r[D][2], v[D][2], x[2], zc = 0.0, ze = 0.0;
+        // the extra tile: of R' for the low strips, of T' for the others
+        const int jx = TM::blk(i, D);
+        const double* const Bx = low ? Y : Tm;
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+          const double2 a = TM::ld(R, i, TM::blk(i, d));
+          r[d][0] = a.x;
+          r[d][1] = a.y;
+          v[d][0] = v[d][1] = 0.0;
+        }
+        x[0] = x[1] = 0.0;
+        if (low) {
+          const double2 a = TM::ld(R, i, jx);
+          x[0] = a.x;
+          x[1] = a.y;
+        }
+#pragma unroll
+        for (int u = 0; u < NB; u++) {
+#pragma unroll
+          for (int d = 0; d < D; d++) {
+            const double2 by = TM::ld(Y, TM::blk(i, d), u), bt = TM::ld(Tm, TM::blk(i, d), u);
+            dmma(r[d], W[u][0], by.x);
+            dmma(v[d], W[u][0], bt.x);
+            dmma(r[d], W[u][1], by.y);
+            dmma(v[d], W[u][1], bt.y);
+          }
+          const double2 bx = TM::ld(Bx, jx, u);
+          dmma(x, W[u][0], bx.x);
+          dmma(x, W[u][1], bx.y);
+          const double2 vc = *reinterpret_cast<const double2*>(S.UC + 8 * u + 2 * q);
+          const double2 ve = *reinterpret_cast<const double2*>(S.UE + 8 * u + 2 * q);
+          zc = fma(W[u][1], vc.y, fma(W[u][0], vc.x, zc));
+          ze = fma(W[u][1], ve.y, fma(W[u][0], ve.x, ze));
+        }
+        zc = quad_sum(zc);
+        ze = quad_sum(ze);
+        team_sync();
+        fro = 0.0;
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+          TM::st_sym(R, i, TM::blk(i, d), r[d]);
+          TM::st_sym(Tm, i, TM::blk(i, d), v[d]);
+          fro += (d == 0 ? 1.0 : 2.0) * (r[d][0] * r[d][0] + r[d][1] * r[d][1]);
+        }
+        TM::st_sym(low ? R : Tm, i, jx, x);
+        if (low) fro += 2.0 * (x[0] * x[0] + x[1] * x[1]);
+        if (q == 0) {
+          const double cc = S.C[row], cn = cc + zc, on = S.o[row] + (0.5 * f) * cc + ze;
+          S.C[row] = cn;
+          S.o[row] = on;
+          S.E[row] = on - f * cn;  // the next step's f is twice this one's
+        }
+        fro = warp_sum(fro);
+        if (lane == 0) S.fro[i] = fro;
+      }
+      tiles += 3 * (NB * (NB + 1) / 2) + NB * NB;
+      even = even + 0.5 * f;
+      f = 2.0 * f;
+    }
+    team_sync();
+    // unscaled R, T, S+ and S- (the layout k_adding reads)
+    {
+      double* out = w.lay + (size_t)item * w.lay_stride;
+      for (int e = t; e < n * n; e += T) {
+        const int col = e / n, r = e % n;
+        const double s = (r == col) ? 1.0 : S.is[r] * S.sc[col];
+        out[col * LD + r] = s * R[TM::at(r, col)];
+        out[LMAT + col * LD + r] = s * Tm[TM::at(r, col)];
+      }
+      for (int e = t; e < n; e += T) {
+        const double m = even * S.C[e], o = S.o[e];
+        out[2 * LMAT + e] = (m + o) * S.is[e];
+        out[2 * LMAT + n + e] = (m - o) * S.is[e];
+      }
+    }
     if (t == 0) {
       w.lay_nd[item] = nd;
       if (status) atomicOr(&w.status[(size_t)c * Fm + fi], status);
+      // products of n x n matrices by the multiply-adds issued (a symmetric one counts its computed tiles)
+      const int nprod = (tiles + NB * NB / 2) / (NB * NB);
       if (nprod) atomicAdd(reinterpret_cast<unsigned long long*>(w.counters + COUNTER_PRODUCTS),
                            (unsigned long long)nprod);
     }
