@@ -3,7 +3,7 @@
 // as 3xTF32 tcgen05 MMAs with FP32 accumulation; the (I - R1+ R2)^-1 solve of
 // every combine stays FP64 (Neumann series on the FP64 tensor path or
 // Gauss-Jordan), and so do the source vectors, the surface coupling and the
-// internal radiances (k_adding_finish, the FP64 code of k_adding).
+// radiances (k_adding_finish, the FP64 code of k_adding).
 //
 // Per (column, frequency) unit the stack (R+, R-, T+, T-) is held in FP32
 // masters in shared memory.  With G = (I - R1+ R2)^-1 a combine is five MMA
@@ -35,6 +35,7 @@
 // combine's last pass runs, into the buffers of W and Y (free once that pass
 // has its operands); the buffer roles rotate every combine.
 #pragma once
+#include "adding.cuh"
 #include "layer_tc.cuh"
 
 namespace pb {
@@ -152,9 +153,8 @@ __device__ __forceinline__ int next_scat(const Batch& b, const Work& w, int c, i
 
 // One unit's n = 32 FP64 product by its two warps (wl = 0, 1 owns rows
 // 16 wl .. 16 wl + 15): C = A B (MM_SET), D + A B (MM_ACC) or I + A B
-// (MM_IPLUS), with the fragments and k order of mm(), so the results are
-// bit-identical to it.  With INPLACE the unit synchronises between reading
-// the operands and writing C.
+// (MM_IPLUS).  With INPLACE the unit synchronises between reading the operands
+// and writing C.
 template <int MODE, bool INPLACE>
 __device__ __forceinline__ void mm_unit(const double* A, const double* B, double* C, const double* D, int wl, int mi) {
   constexpr int LD = Team<32>::LD;
@@ -590,45 +590,51 @@ __global__ void __launch_bounds__(128, 2) k_adding_tc(Batch b, Work w, pamtra_b2
   if (warp == 0) tc::tmem_dealloc(tslot, 128);
 }
 
-// Surface, internal radiances and TB of the units k_adding_tc carried, in
-// FP64 from their FP32 stacks (the code of k_adding after its layer loop).
+// Surface, radiances and TB of the units k_adding_tc carried, in FP64 from
+// their FP32 stacks (the end of k_adding).
 template <int N>
-__global__ void __launch_bounds__(RTCfg<N>::T) k_adding_finish(Batch b, Work w, pamtra_b200_settings st,
-                                                               pamtra_b200_outputs out) {
-  constexpr int n = RTCfg<N>::n, LD = RTCfg<N>::LD, T = RTCfg<N>::T;
+__global__ void __launch_bounds__(SymTeam<2 * N>::T) k_adding_finish(Batch b, Work w, pamtra_b200_settings st,
+                                                                     pamtra_b200_outputs out) {
+  using A = Adder<N, false>;
+  using TM = SymTeam<2 * N>;
+  constexpr int n = 2 * N, T = TM::T, NB = TM::NB;
   extern __shared__ double smem_raw[];
   AddSmem<N>& S = *reinterpret_cast<AddSmem<N>*>(smem_raw);
-  const int t = threadIdx.x;
+  const int t = threadIdx.x, lane = t & 31, i = t >> 5;
   const int Fm = b.max_nfreq;
   const int nunits = b.ncol * Fm;
-  if (t < N) { S.mu[t] = w.lob_mu[lob_off(N) + t]; S.wq[t] = w.lob_w[lob_off(N) + t]; }
+  A::init(S, w);
   for (int unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
     const int c = unit / Fm, fi = unit % Fm;
     if (fi >= b.col_nfreq(c) || b.col_nummu(c) != N) continue;
     const float* stk = w.add_stk + (size_t)unit * STK_FLOATS;
     const int sstate = reinterpret_cast<const int*>(stk + STK_HDR)[0];
     const int status = reinterpret_cast<const int*>(stk + STK_HDR)[1];
-    double *Rp = S.m[0], *Rm = S.m[1], *Tp = S.m[2], *Tm = S.m[3];
+    typename A::RG G;
+    team_sync();
     if (sstate == 2) {
       for (int s = t; s < 1024; s += T) {
         int r, cc;
         midx_inv(s, r, cc);
-        Rp[cc * LD + r] = stk[STK_RP + s];
-        Rm[cc * LD + r] = stk[STK_RM + s];
-        Tp[cc * LD + r] = stk[STK_TP + s];
-        Tm[cc * LD + r] = stk[STK_TM + s];
+        S.m[0][TM::at(r, cc)] = stk[STK_RP + s];
+        S.m[1][TM::at(r, cc)] = stk[STK_TP + s];
       }
+#pragma unroll
+      for (int j = 0; j < NB; j++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int s = midx(8 * i + (lane >> 2), 8 * j + 2 * (lane & 3) + e);
+          G.rm[j][e] = stk[STK_RM + s];
+          G.tm[j][e] = stk[STK_TM + s];
+        }
     }
     if (t < n) {
-      S.sp[t] = stk[STK_SP + t];
-      S.sm[t] = stk[STK_SM + t];
-      S.t1[t] = stk[STK_T1 + t];
+      S.sp[t] = S.cp[t] = sstate ? stk[STK_SP + t] : 0.0;
+      S.sm[t] = S.cm[t] = sstate ? stk[STK_SM + t] : 0.0;
+      S.tc[t] = sstate ? stk[STK_T1 + t] : 1.0;
     }
     team_sync();
-    const double wl = C_LIGHT / (b.freq(c, fi) * 1.e3);
-    adding_finish<N>(b, w, st, out, S, c, fi, b.nlyrs[c], wl, sstate, status, Rp, Rm, Tp, Tm, S.m[4], S.m[5],
-                     S.m[6], S.m[7], S.m[8]);
-    team_sync();
+    A::finish(b, w, st, out, S, G, i, c, fi, sstate == 2, status);
   }
 }
 

@@ -22,6 +22,7 @@
 #include "mie.cuh"
 #include "prep.cuh"
 #include "rt.cuh"
+#include "adding.cuh"
 #include "tc.cuh"
 #include "layer_tc.cuh"
 #include "layer_tc64.cuh"
@@ -239,11 +240,10 @@ struct Plan {
   size_t o_slot_st, o_slot_nb, o_bd, o_bdd, o_bnd, o_brho, o_bmass;
   size_t o_pres_idx, o_plist, o_counters, o_mkext, o_msalb, o_mback, o_mrefr, o_mnleg, o_mlegen, o_lay, o_laynd, o_status,
       o_colst, o_colcnt;
-  size_t o_species, o_addscr, o_mieslab, o_addstk;
+  size_t o_species, o_segcnt, o_mieslab, o_addstk;
   int mie_nslab;  // k_mie warps the slabs are sized for
   bool f32_coef;
   bool tc_add;  // split-precision adding for NUMMU 16 (FP32 layer records, stacks)
-  int add_grid;  // CTAs of k_adding<32> the scratch is sized for
   int pmax;
   int max_nbin;
   int maxN;
@@ -309,8 +309,7 @@ Plan make_plan(const pamtra_b200_columns* c, int default_nummu, int sms, int mie
   p.o_colst = take(C * 4);
   p.o_colcnt = take(C * 4);
   p.o_species = take(std::max<size_t>(nsp, 1) * sizeof(pamtra_b200_species));
-  p.add_grid = (mask & 4) ? std::max(1, sms) : 0;
-  p.o_addscr = take((size_t)p.add_grid * (10 - AddSmem<32>::NS) * RTCfg<32>::MAT * 8);
+  p.o_segcnt = take(C * Fm * 4);
   // one slab per k_mie warp; more warps than (layer, frequency) items would idle
   p.mie_nslab = c->nhydro > 0 ? (int)std::min<size_t>((size_t)mie_slabs, items) : 0;
   p.o_mieslab = take((size_t)p.mie_nslab * MIE_SLAB_STRIDE * 8);
@@ -331,6 +330,13 @@ int occupancy_blocks(const void* func, int threads, size_t smem, int sms) {
 int persistent_grid(const void* func, int threads, size_t smem, int sms, int cps) {
   const int full = occupancy_blocks(func, threads, smem, sms);
   return cps > 0 ? std::min(full, cps * sms) : full;
+}
+
+template <int N, bool SYM>
+void launch_adding(const Batch& b, const Work& w, const pamtra_b200_settings& st, const pamtra_b200_outputs& out,
+                   int maxseg, int sms, int cps, cudaStream_t stream) {
+  const int g = persistent_grid((const void*)k_adding<N, SYM>, SymTeam<2 * N>::T, sizeof(AddSmem<N>), sms, cps);
+  k_adding<N, SYM><<<g, SymTeam<2 * N>::T, sizeof(AddSmem<N>), stream>>>(b, w, st, out, maxseg);
 }
 
 }  // namespace
@@ -514,12 +520,11 @@ static int set_smem_attrs() {
     set((const void*)k_layer<32>, sizeof(LayerSmem<32>));
     set((const void*)k_layer_tc<16>, layer_tc_smem<16>());
     set((const void*)k_layer_tc64, layer_tc64_smem());
-    set((const void*)k_adding<8>, sizeof(AddSmem<8>));
-    set((const void*)k_adding<16>, sizeof(AddSmem<16>));
-    set((const void*)k_adding<32>, sizeof(AddSmem<32>));
     set((const void*)k_adding<8, true>, sizeof(AddSmem<8>));
     set((const void*)k_adding<16, true>, sizeof(AddSmem<16>));
+    set((const void*)k_adding<16, false>, sizeof(AddSmem<16>));
     set((const void*)k_adding<32, true>, sizeof(AddSmem<32>));
+    set((const void*)k_adding<32, false>, sizeof(AddSmem<32>));
     set((const void*)k_minvert<64>, Team<64>::MAT * 8 + sizeof(InvScratch<64>));
     set((const void*)k_adding_tc<16>, add_tc_smem());
     set((const void*)k_adding_finish<16>, sizeof(AddSmem<16>));
@@ -771,7 +776,6 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   if (precision != PAMTRA_B200_PREC_FP64 && precision != PAMTRA_B200_PREC_3XTF32 &&
       precision != PAMTRA_B200_PREC_FP64_BATCHED && precision != PAMTRA_B200_PREC_3XTF32_FP64ADD)
     return PAMTRA_B200_FATAL;
-  const bool one_inv = precision != PAMTRA_B200_PREC_FP64;  // one inverse per adding combine
   // split precision: 3xTF32 doubling (and, for PREC_3XTF32, adding of NUMMU 16)
   const bool split = precision == PAMTRA_B200_PREC_3XTF32 || precision == PAMTRA_B200_PREC_3XTF32_FP64ADD;
   if (cols->ncol < 1 || cols->max_nlyrs < 2 || cols->max_nfreq < 1 || cols->noutlevels < 1 || cols->nhydro < 0)
@@ -865,7 +869,7 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   w.lay32 = pl.tc_add ? 1 : 0;
   w.add_stk = pl.tc_add ? (float*)(A + pl.o_addstk) : nullptr;
   w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst); w.col_cnt = (int*)(A + pl.o_colcnt);
-  w.add_scr = (double*)(A + pl.o_addscr);
+  w.seg_cnt = (int*)(A + pl.o_segcnt);
   w.mie_slab = (double*)(A + pl.o_mieslab); w.mie_nslab = pl.mie_nslab;
   w.spin_limit = ctx->spin_limit;
   ctx->last_counters = w.counters;
@@ -894,6 +898,8 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   cudaMemsetAsync(w.counters, 0, 16 * 4, stream);
   cudaMemsetAsync(w.status, 0, C * Fm * 4, stream);
   cudaMemsetAsync(w.col_status, 0, C * 4, stream);
+  cudaMemsetAsync(w.seg_cnt, 0, C * Fm * 4, stream);
+  const int maxseg = add_max_segments((int)Lm);
   const size_t ntb = C * cc.noutlevels * 2 * cc.max_nummu * Fm * 2;
   k_fill_d<<<(unsigned)((ntb + 255) / 256), 256, 0, stream>>>(out->tb, -9999.0, ntb); launches++;
   if (w.psd_d && H > 0) {
@@ -947,9 +953,7 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
     int g = persistent_grid((const void*)k_layer<8>, LayerCfg<8>::T, sizeof(LayerSmem<8>), sms, ctx->layer_cps);
     if (H > 0) { k_layer<8><<<g, LayerCfg<8>::T, sizeof(LayerSmem<8>), stream>>>(b, w, *st, ssp); launches++; }
     mark(ctx, stream, STG_LAYER);
-    g = persistent_grid((const void*)k_adding<8>, RTCfg<8>::T, sizeof(AddSmem<8>), sms, ctx->adding_cps);
-    if (one_inv) k_adding<8, true><<<g, RTCfg<8>::T, sizeof(AddSmem<8>), stream>>>(b, w, *st, *out);
-    else k_adding<8><<<g, RTCfg<8>::T, sizeof(AddSmem<8>), stream>>>(b, w, *st, *out);
+    launch_adding<8, true>(b, w, *st, *out, maxseg, sms, ctx->adding_cps, stream);
     launches++;
     mark(ctx, stream, STG_ADDING);
   }
@@ -970,13 +974,12 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
       // two CTAs (two unit pairs) per SM by shared memory and tensor memory
       // (2 x 256 columns); the FP64 surface and radiance part follows
       k_adding_tc<16><<<2 * sms, 128, add_tc_smem(), stream>>>(b, w, *st);
-      const int gf = persistent_grid((const void*)k_adding_finish<16>, RTCfg<16>::T, sizeof(AddSmem<16>), sms, 0);
-      k_adding_finish<16><<<gf, RTCfg<16>::T, sizeof(AddSmem<16>), stream>>>(b, w, *st, *out);
+      const int gf = persistent_grid((const void*)k_adding_finish<16>, SymTeam<32>::T, sizeof(AddSmem<16>), sms, 0);
+      k_adding_finish<16><<<gf, SymTeam<32>::T, sizeof(AddSmem<16>), stream>>>(b, w, *st, *out);
       launches += 2;
     } else {
-      const int g = persistent_grid((const void*)k_adding<16>, RTCfg<16>::T, sizeof(AddSmem<16>), sms, ctx->adding_cps);
-      if (one_inv) k_adding<16, true><<<g, RTCfg<16>::T, sizeof(AddSmem<16>), stream>>>(b, w, *st, *out);
-      else k_adding<16><<<g, RTCfg<16>::T, sizeof(AddSmem<16>), stream>>>(b, w, *st, *out);
+      if (split) launch_adding<16, false>(b, w, *st, *out, maxseg, sms, ctx->adding_cps, stream);
+      else launch_adding<16, true>(b, w, *st, *out, maxseg, sms, ctx->adding_cps, stream);
       launches++;
     }
     mark(ctx, stream, STG_ADDING);
@@ -990,10 +993,8 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
       k_layer<32><<<g, LayerCfg<32>::T, sizeof(LayerSmem<32>), stream>>>(b, w, *st, ssp); launches++;
     }
     mark(ctx, stream, STG_LAYER);
-    g = std::min(persistent_grid((const void*)k_adding<32>, RTCfg<32>::T, sizeof(AddSmem<32>), sms, ctx->adding_cps),
-                 pl.add_grid);
-    if (one_inv) k_adding<32, true><<<g, RTCfg<32>::T, sizeof(AddSmem<32>), stream>>>(b, w, *st, *out);
-    else k_adding<32><<<g, RTCfg<32>::T, sizeof(AddSmem<32>), stream>>>(b, w, *st, *out);
+    if (split) launch_adding<32, false>(b, w, *st, *out, maxseg, sms, ctx->adding_cps, stream);
+    else launch_adding<32, true>(b, w, *st, *out, maxseg, sms, ctx->adding_cps, stream);
     launches++;
     mark(ctx, stream, STG_ADDING);
   }
@@ -1444,6 +1445,7 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   w.m_legen32 = pl.f32_coef ? (float*)(A + pl.o_mlegen) : nullptr;
   w.lay = (double*)(A + pl.o_lay); w.lay_stride = pl.lay_stride; w.lay_nd = (int*)(A + pl.o_laynd);
   w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst); w.col_cnt = (int*)(A + pl.o_colcnt);
+  w.seg_cnt = (int*)(A + pl.o_segcnt);
   w.spin_limit = tc::MBAR_SPIN_LIMIT;
   w.mie_slab = (double*)(A + pl.o_mieslab); w.mie_nslab = pl.mie_nslab;
   w.gq_x = D.tables; w.gq_w = D.tables + gqn; w.gq_max = NOALLOC_GQ;
@@ -1453,6 +1455,8 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   cudaMemsetAsync(w.counters, 0, 16 * 4, stream);
   cudaMemsetAsync(w.status, 0, Fm * 4, stream);
   cudaMemsetAsync(w.col_status, 0, 4, stream);
+  cudaMemsetAsync(w.seg_cnt, 0, Fm * 4, stream);
+  const int maxseg = add_max_segments((int)Lm);
   const size_t ntb = (size_t)cc.noutlevels * 2 * cc.max_nummu * Fm * 2;
   k_fill_d<<<(unsigned)((ntb + 255) / 256), 256, 0, stream>>>(out->tb, -9999.0, ntb);
   k_atmo<<<1, 128, 0, stream>>>(b, w);
@@ -1468,11 +1472,11 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   }
   if (mask & 1) {
     if (nh > 0) k_layer<8><<<sms, LayerCfg<8>::T, sizeof(LayerSmem<8>), stream>>>(b, w, *st, out->scatter_matrix);
-    k_adding<8><<<sms, RTCfg<8>::T, sizeof(AddSmem<8>), stream>>>(b, w, *st, *out);
+    launch_adding<8, true>(b, w, *st, *out, maxseg, sms, 1, stream);
   }
   if (mask & 2) {
     if (nh > 0) k_layer<16><<<sms, LayerCfg<16>::T, sizeof(LayerSmem<16>), stream>>>(b, w, *st, out->scatter_matrix);
-    k_adding<16><<<sms, RTCfg<16>::T, sizeof(AddSmem<16>), stream>>>(b, w, *st, *out);
+    launch_adding<16, true>(b, w, *st, *out, maxseg, sms, 1, stream);
   }
   if (out->angles_deg) k_angles<<<1, 32, 0, stream>>>(out->angles_deg, w.lob_mu, cc.max_nummu);
   if (out->kexttot || out->salbedo || out->num_doubles)

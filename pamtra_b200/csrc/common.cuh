@@ -111,124 +111,8 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// An 8 x 8 accumulator tile (row block i, column block j) to and from a
-// column-major matrix.  A lane holds row g of columns 2q and 2q + 1; with
-// LD = 4 mod 16 the lanes of q and q + 2 meet in a bank when all lanes take
-// column 2q first, so q >= 2 takes 2q + 1 first: two wavefronts per access, the least
-// for 32 doubles, instead of four.
-template <int n>
-__device__ __forceinline__ void store_tile(double* C, int i, int j, const double (&c)[2]) {
-  constexpr int LD = Team<n>::LD;
-  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, o = q >> 1;
-  double* p = C + (8 * j + 2 * q) * LD + 8 * i + g;
-  p[o * LD] = o ? c[1] : c[0];
-  p[(1 - o) * LD] = o ? c[0] : c[1];
-}
-template <int n>
-__device__ __forceinline__ void load_tile(const double* C, int i, int j, double (&c)[2]) {
-  constexpr int LD = Team<n>::LD;
-  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3, o = q >> 1;
-  const double* p = C + (8 * j + 2 * q) * LD + 8 * i + g;
-  const double x = p[o * LD], y = p[(1 - o) * LD];
-  c[0] = o ? y : x;
-  c[1] = o ? x : y;
-}
-
-enum MMMode { MM_SET = 0, MM_ACC = 1, MM_IMINUS = 2, MM_IPLUS = 3 };
-
-// C = A*B (MM_SET), C = D + A*B (MM_ACC), C = I - A*B (MM_IMINUS) or
-// C = I + A*B (MM_IPLUS).
-// Each warp computes one 16 x 16 tile with 2 x 2 DMMA fragments per k-step
-// of 4.  Without INPLACE, C must not alias A or B; with INPLACE the team
-// synchronises between reading the operands and writing C, so C may be A,
-// B or D.
-template <int n, int MODE, bool INPLACE = false>
-__device__ __forceinline__ void mm(const double* A, const double* B, double* C, const double* D = nullptr) {
-  constexpr int LD = Team<n>::LD, WT = n / 16;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int row0 = (warp / WT) * 16, col0 = (warp % WT) * 16;
-  const int g = lane >> 2, q = lane & 3;
-  double c[2][2][2];
-#pragma unroll
-  for (int rt = 0; rt < 2; rt++)
-#pragma unroll
-    for (int ct = 0; ct < 2; ct++)
-#pragma unroll
-      for (int i = 0; i < 2; i++) {
-        const int row = row0 + rt * 8 + g, col = col0 + ct * 8 + 2 * q + i;
-        c[rt][ct][i] = (MODE == MM_IMINUS || MODE == MM_IPLUS) ? (row == col ? 1.0 : 0.0) : 0.0;
-      }
-  if (MODE == MM_ACC)
-#pragma unroll
-    for (int rt = 0; rt < 2; rt++)
-#pragma unroll
-      for (int ct = 0; ct < 2; ct++) load_tile<n>(D, (row0 >> 3) + rt, (col0 >> 3) + ct, c[rt][ct]);
-  const double sgn = (MODE == MM_IMINUS) ? -1.0 : 1.0;
-#pragma unroll 4
-  for (int kk = 0; kk < n; kk += 4) {
-    const double a0 = sgn * A[(kk + q) * LD + row0 + g];
-    const double a1 = sgn * A[(kk + q) * LD + row0 + 8 + g];
-    const double b0 = B[(col0 + g) * LD + kk + q];
-    const double b1 = B[(col0 + 8 + g) * LD + kk + q];
-    dmma(c[0][0], a0, b0);
-    dmma(c[0][1], a0, b1);
-    dmma(c[1][0], a1, b0);
-    dmma(c[1][1], a1, b1);
-  }
-  if (INPLACE) team_sync();
-#pragma unroll
-  for (int rt = 0; rt < 2; rt++)
-#pragma unroll
-    for (int ct = 0; ct < 2; ct++) store_tile<n>(C, (row0 >> 3) + rt, (col0 >> 3) + ct, c[rt][ct]);
-}
-
-// Two products with the same left factor in one pass over K:
-// C1 = A B1 (+ D1) and C2 = A B2 (+ D2), modes MM_SET / MM_ACC each.  The A
-// fragments are loaded once for both (six operand loads per k-step for eight
-// DMMAs instead of eight), and each element accumulates in the same order as
-// in mm(), so the results are bit-identical to two mm() calls.  C1 and C2
-// must not alias A, B1 or B2.
-template <int n, int MODE1, int MODE2>
-__device__ __forceinline__ void mm2(const double* A, const double* B1, double* C1, const double* D1,
-                                    const double* B2, double* C2, const double* D2) {
-  constexpr int LD = Team<n>::LD, WT = n / 16;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int row0 = (warp / WT) * 16, col0 = (warp % WT) * 16;
-  const int g = lane >> 2, q = lane & 3;
-  double c[2][2][2], e[2][2][2];
-#pragma unroll
-  for (int rt = 0; rt < 2; rt++)
-#pragma unroll
-    for (int ct = 0; ct < 2; ct++) {
-      c[rt][ct][0] = c[rt][ct][1] = e[rt][ct][0] = e[rt][ct][1] = 0.0;
-      if (MODE1 == MM_ACC) load_tile<n>(D1, (row0 >> 3) + rt, (col0 >> 3) + ct, c[rt][ct]);
-      if (MODE2 == MM_ACC) load_tile<n>(D2, (row0 >> 3) + rt, (col0 >> 3) + ct, e[rt][ct]);
-    }
-#pragma unroll 4
-  for (int kk = 0; kk < n; kk += 4) {
-    const double a0 = A[(kk + q) * LD + row0 + g];
-    const double a1 = A[(kk + q) * LD + row0 + 8 + g];
-    const double b0 = B1[(col0 + g) * LD + kk + q];
-    const double b1 = B1[(col0 + 8 + g) * LD + kk + q];
-    const double f0 = B2[(col0 + g) * LD + kk + q];
-    const double f1 = B2[(col0 + 8 + g) * LD + kk + q];
-    dmma(c[0][0], a0, b0);
-    dmma(e[0][0], a0, f0);
-    dmma(c[0][1], a0, b1);
-    dmma(e[0][1], a0, f1);
-    dmma(c[1][0], a1, b0);
-    dmma(e[1][0], a1, f0);
-    dmma(c[1][1], a1, b1);
-    dmma(e[1][1], a1, f1);
-  }
-#pragma unroll
-  for (int rt = 0; rt < 2; rt++)
-#pragma unroll
-    for (int ct = 0; ct < 2; ct++) {
-      store_tile<n>(C1, (row0 >> 3) + rt, (col0 >> 3) + ct, c[rt][ct]);
-      store_tile<n>(C2, (row0 >> 3) + rt, (col0 >> 3) + ct, e[rt][ct]);
-    }
-}
+// C = A B, C = D + A B, C = I + A B
+enum MMMode { MM_SET = 0, MM_ACC = 1, MM_IPLUS = 2 };
 
 // ------------------------------------------------------------------ symmetric-matrix teams
 // A team of n / 8 warps works on symmetric n x n matrices (and one general
@@ -287,16 +171,6 @@ struct SymTeam {
   // results of a pass, so every strip has NB + 1 tiles of a pair).
   __device__ static __forceinline__ int blk(int i, int d) { return (i + d) & (NB - 1); }
 };
-
-// row `row` of M * x (k-ascending FMA chain)
-template <int n>
-__device__ __forceinline__ double mv_row(const double* __restrict__ M, const double* __restrict__ x, int row) {
-  constexpr int LD = Team<n>::LD;
-  double s = 0.0;
-#pragma unroll 8
-  for (int k = 0; k < n; k++) s = fma(M[k * LD + row], x[k], s);
-  return s;
-}
 
 // Scratch of the inverse routines.
 template <int n>
@@ -406,83 +280,6 @@ __device__ int ginv(double* A, InvScratch<n>& S) {
   for (int jj = 0; jj < NC; jj++) A[(cg + CG * jj) * LD + i] = col[jj];
   team_sync();
   return S.sing;
-}
-
-// G = (I - X)^-1 in FP64.  X (in buffer P) is overwritten.  When the row-sum
-// norm of X is below 0.74 the inverse is a truncated Neumann series whose
-// remainder is below 2^-54 relative (the FP64 rounding unit), evaluated with
-// the fewer products of two forms:
-//   Horner    G = I + X (I + X (... (I + X)))   k products, remainder ||X||^(k+2)
-//   squaring  G = (I + X)(I + X^2)(I + X^4)...  2 (m-1) products, remainder ||X||^(2^m)
-// (Horner wins for the thin layers of the first doublings, where ||X|| is
-// tiny and G = I + X needs no product at all); otherwise Gauss-Jordan with
-// partial pivoting.  Returns the buffer holding the inverse (P or G); *sing
-// set on a zero pivot.
-template <int n>
-__device__ double* inv_iminus(double* P, double* G, InvScratch<n>& S, int* sing) {
-  constexpr int LD = Team<n>::LD, T = Team<n>::T;
-  const int t = threadIdx.x;
-  // infinity norm of X
-  if (t < n) {
-    double r = 0.0;
-#pragma unroll 8
-    for (int j = 0; j < n; j++) r += fabs(P[j * LD + t]);
-    const unsigned mask = (n >= 32) ? 0xffffffffu : ((1u << n) - 1u);
-#pragma unroll
-    for (int o = ((n >= 32) ? 16 : n / 2); o > 0; o >>= 1) r = fmax(r, __shfl_xor_sync(mask, r, o));
-    if ((t & 31) == 0) S.cand_v[t >> 5] = r;
-  }
-  team_sync();
-  double nrm = S.cand_v[0];
-#pragma unroll
-  for (int w = 1; w < (n + 31) / 32; w++) nrm = fmax(nrm, S.cand_v[w]);
-  int m = 1;
-  double pw = nrm;
-  while (pw > 5.0e-17 && m < 8) {
-    pw = pw * pw;
-    m++;
-  }
-  int kh = 0;  // Horner products
-  double ph = nrm * nrm;
-  while (ph > 5.0e-17 && kh < 2 * (m - 1)) {
-    ph = ph * nrm;
-    kh++;
-  }
-  if (m < 8 && ph <= 5.0e-17 && kh < 2 * (m - 1)) {
-    for (int e = t; e < n * n; e += T) {
-      const int col = e / n, row = e % n;
-      G[col * LD + row] = ((row == col) ? 1.0 : 0.0) + P[col * LD + row];
-    }
-    team_sync();
-    for (int k = 0; k < kh; k++) {
-      mm<n, MM_IPLUS, true>(P, G, G);  // G = I + X G
-      team_sync();
-    }
-    return G;
-  }
-  if (m >= 8) {
-    // Gauss-Jordan on I - X
-    for (int e = t; e < n * n; e += T) {
-      const int col = e / n, row = e % n;
-      P[col * LD + row] = ((row == col) ? 1.0 : 0.0) - P[col * LD + row];
-    }
-    team_sync();
-    if (ginv<n>(P, S)) *sing = 1;
-    return P;
-  }
-  // G = I + X
-  for (int e = t; e < n * n; e += T) {
-    const int col = e / n, row = e % n;
-    G[col * LD + row] = ((row == col) ? 1.0 : 0.0) + P[col * LD + row];
-  }
-  team_sync();
-  for (int k = 1; k < m; k++) {
-    mm<n, MM_SET, true>(P, P, P);     // P = P^2
-    team_sync();
-    mm<n, MM_ACC, true>(G, P, G, G);  // G = G + G P
-    team_sync();
-  }
-  return G;
 }
 
 }  // namespace pb

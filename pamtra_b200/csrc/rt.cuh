@@ -3,11 +3,9 @@
 //     series -> quadrature phase matrices), check_norm4, INITIALIZE4 /
 //     INITIAL_SOURCE4 and DOUBLING_INTEGRATION4; writes the layer's R, T and
 //     S+/S- to the scratch arena.
-//   k_adding<N>: per (column, frequency) unit -- adding of all layers top
-//     down (COMBINE_LAYERS4 specialised by structure), surface, internal
-//     radiance at the output levels and conversion to brightness temperature.
-// Both are persistent kernels: one CTA ("team", see common.cuh) per item,
-// items taken from a device-side counter.
+// The adding of a column's layers is in adding.cuh.  Both are persistent
+// kernels: one CTA ("team", see common.cuh) per item, items taken from a
+// device-side counter.
 #pragma once
 #include "common.cuh"
 #include "work.cuh"
@@ -375,7 +373,8 @@ __device__ __forceinline__ bool layer_setup(const Batch& b, const Work& w, const
   return true;
 }
 
-// Write the layer R, T and S+/S- of an item (FP64, the layout k_adding reads).
+// Write the layer R, T and S+/S- of an item (FP64, unscaled, column-major with
+// leading dimension n + 4: what k_adding<N, false> reads).
 template <int N, int T = RTCfg<N>::T>
 __device__ __forceinline__ void layer_store(const Work& w, int item, const double* Rb, const double* Tb,
                                             const double* lin) {
@@ -425,7 +424,7 @@ __global__ void __launch_bounds__(LayerCfg<N>::T, LayerCfg<N>::CTAS) k_layer(Bat
                                                                             double* __restrict__ ssp_scat) {
   using TM = SymTeam<2 * N>;
   constexpr int n = 2 * N, T = TM::T, NB = TM::NB, D = TM::D;
-  constexpr int LD = RTCfg<N>::LD, LMAT = RTCfg<N>::MAT;  // layout of layer_setup, the elimination and the layer records
+  constexpr int LD = RTCfg<N>::LD;  // leading dimension of layer_setup's matrices and the elimination
   extern __shared__ double smem_raw[];
   LayerSmem<N>& S = *reinterpret_cast<LayerSmem<N>*>(smem_raw);
   const int t = threadIdx.x, lane = t & 31, i = t >> 5;  // i: this warp's strip
@@ -711,19 +710,19 @@ __global__ void __launch_bounds__(LayerCfg<N>::T, LayerCfg<N>::CTAS) k_layer(Bat
       f = 2.0 * f;
     }
     team_sync();
-    // unscaled R, T, S+ and S- (the layout k_adding reads)
+    // the layer record k_adding<N, true> reads: the scaled R and T as they lie, S+ and S-
     {
       double* out = w.lay + (size_t)item * w.lay_stride;
-      for (int e = t; e < n * n; e += T) {
-        const int col = e / n, r = e % n;
-        const double s = (r == col) ? 1.0 : S.is[r] * S.sc[col];
-        out[col * LD + r] = s * R[TM::at(r, col)];
-        out[LMAT + col * LD + r] = s * Tm[TM::at(r, col)];
+      const double2 *r2 = reinterpret_cast<const double2*>(R), *t2 = reinterpret_cast<const double2*>(Tm);
+      double2* o2 = reinterpret_cast<double2*>(out);
+      for (int e = t; e < n * n / 2; e += T) {
+        o2[e] = r2[e];
+        o2[n * n / 2 + e] = t2[e];
       }
       for (int e = t; e < n; e += T) {
         const double m = even * S.C[e], o = S.o[e];
-        out[2 * LMAT + e] = (m + o) * S.is[e];
-        out[2 * LMAT + n + e] = (m - o) * S.is[e];
+        out[2 * n * n + e] = m + o;
+        out[2 * n * n + n + e] = m - o;
       }
     }
     if (t == 0) {
@@ -734,469 +733,6 @@ __global__ void __launch_bounds__(LayerCfg<N>::T, LayerCfg<N>::CTAS) k_layer(Bat
       if (nprod) atomicAdd(reinterpret_cast<unsigned long long*>(w.counters + COUNTER_PRODUCTS),
                            (unsigned long long)nprod);
     }
-  }
-}
-
-// ============================================================== adding kernel
-// Ten n x n matrices per column-frequency unit.  For N <= 16 all of them live
-// in shared memory; for N = 32 (n = 64, 34 KB per matrix) the first six do and
-// the last four (G, X, Y, Z) live in a per-CTA slice of global scratch
-// (Work::add_scr), which stays L2-resident.
-template <int N>
-struct AddSmem {
-  static constexpr int n = RTCfg<N>::n, MAT = RTCfg<N>::MAT;
-  static constexpr int NS = (N == 32) ? 6 : 10;  // matrices in shared memory
-  double m[NS][MAT];
-  double sp[n], sm[n], s2p[n], s2m[n], t1[n], t2[n], nsp[n], nsm[n];
-  double wv[n], wv2[n], u1[n], u2[n];
-  double sky[n], gnd[n], uprad[n], dnrad[n];
-  double mu[N], wq[N];
-  InvScratch<n> inv;
-  int unit;
-};
-
-template <int n>
-__device__ __forceinline__ void ew_ident(double* A) {  // A = I
-  constexpr int LD = Team<n>::LD, T = Team<n>::T;
-  for (int e = threadIdx.x; e < n * n; e += T) {
-    const int col = e / n, row = e % n;
-    A[col * LD + row] = (row == col) ? 1.0 : 0.0;
-  }
-}
-template <int n>
-__device__ __forceinline__ void ew_zero(double* A) {
-  constexpr int LD = Team<n>::LD, T = Team<n>::T;
-  for (int e = threadIdx.x; e < n * n; e += T) A[(e / n) * LD + e % n] = 0.0;
-}
-template <int n>
-__device__ __forceinline__ void ew_diag(double* A, const double* d) {
-  constexpr int LD = Team<n>::LD, T = Team<n>::T;
-  for (int e = threadIdx.x; e < n * n; e += T) {
-    const int col = e / n, row = e % n;
-    A[col * LD + row] = (row == col) ? d[col] : 0.0;
-  }
-}
-
-// End of the adding for one (column, frequency) unit: the stack (Rp, Rm, Tp,
-// Tm with sources S.sp / S.sm, or a clear stack t1 / sp / sm when sstate <= 1)
-// on the surface, the internal radiances at the output levels, TB, status.
-// R2, T2, G, X, Y are scratch matrices (G and X may be swapped by the
-// inverses).
-template <int N>
-__device__ __forceinline__ void adding_finish(const Batch& b, const Work& w, const pamtra_b200_settings& st,
-                                              const pamtra_b200_outputs& out, AddSmem<N>& S, int c, int fi,
-                                              int L, double wl, int sstate, int status, double* Rp, double* Rm,
-                                              double* Tp, double* Tm, double* R2, double* T2, double* G,
-                                              double* X, double* Y) {
-  constexpr int n = RTCfg<N>::n, LD = RTCfg<N>::LD, MAT = RTCfg<N>::MAT, T = RTCfg<N>::T;
-  const int t = threadIdx.x;
-  const int Fm = b.max_nfreq;
-  // materialise a clear (or empty) stack
-  if (sstate <= 1) {
-    if (sstate == 0 && t < n) { S.t1[t] = 1.0; S.sp[t] = 0.0; S.sm[t] = 0.0; }
-    team_sync();
-    ew_diag<n>(Tp, S.t1);
-    ew_diag<n>(Tm, S.t1);
-    ew_zero<n>(Rp);
-    ew_zero<n>(Rm);
-    team_sync();
-  }
-  // surface (src/sfc_matrices.f90; default emissivity sfc_optics.f90:79-81)
-  // and sky (src/surface.f90:169-195)
-  const char refl = (char)b.sfc_refl[c];
-  const double e = st.emissivity, rr = 1.0 - e;
-  const double pg = planck(w.gtemp[c], wl), psky = planck(SKY_TEMP, wl);
-  for (int ee = t; ee < n * n; ee += T) {  // R2 := surface R- (R+ = 0), T2 := I
-    const int col = ee / n, row = ee % n;
-    double v = 0.0;
-    if (refl == 'S' || refl == 'F') {
-      const double r1 = (rr + rr) / 2.0, r2 = (rr - rr) / 2.0;
-      if ((row >> 1) == (col >> 1)) v = ((row & 1) == (col & 1)) ? r1 : r2;
-    } else if (refl == 'L') {
-      if ((row & 1) == 0 && (col & 1) == 0) v = 2.0 * rr * S.mu[col >> 1] * S.wq[col >> 1];
-    }
-    R2[col * LD + row] = v;
-    T2[col * LD + row] = (row == col) ? 1.0 : 0.0;
-  }
-  if (refl != 'S' && refl != 'F' && refl != 'L') status |= PAMTRA_B200_WARNING;
-  if (t < n) {
-    const int i = t & 1;
-    double gv = 0.0;
-    if (refl == 'S' || refl == 'F') {
-      const double r1 = (rr + rr) / 2.0, r2 = (rr - rr) / 2.0;
-      gv = (i == 0) ? (1.0 - r1) * pg : -r2 * pg;
-    } else if (refl == 'L') {
-      gv = (i == 0) ? e * pg : 0.0;
-    }
-    S.gnd[t] = gv;
-    S.sky[t] = (i == 0) ? (1.0 - 0.0) * psky : 0.0;
-    S.s2m[t] = 0.0;  // the surface carries no source in the adding
-  }
-  team_sync();
-  // output levels: L+1 -> (stack, surface); 1 -> (empty, stack on surface)
-  int lev_order[2] = {-1, -1};
-  for (int io = 0; io < b.noutlevels; io++) {
-    const int lev = w.outlev[(size_t)c * b.noutlevels + io];
-    if (lev == L + 1) lev_order[0] = io;
-    else if (lev == 1) lev_order[1] = io;
-    else status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;  // intermediate levels not supported
-  }
-  for (int pass = 0; pass < 2; pass++) {
-    const int io = lev_order[pass];
-    if (io < 0) continue;
-    if (pass == 1) {
-      // down stack for level 1: (stack) on top of (surface), minus side only
-      mm<n, MM_SET>(R2, Rp, G);  // GAMMAm = inv(I - Rsfc R1p)
-      team_sync();
-      {
-        int sg = 0;
-        double* gi = inv_iminus<n>(G, X, S.inv, &sg);
-        if (sg) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_PIVOT;
-        if (gi != G) { X = G; G = gi; }
-      }
-      mm<n, MM_SET>(R2, Tp, X);
-      if (t < n) S.wv[t] = 0.0 + mv_row<n>(R2, S.sp, t);
-      team_sync();
-      mm<n, MM_SET>(G, X, Y);
-      if (t < n) S.wv2[t] = mv_row<n>(G, S.wv, t);
-      team_sync();
-      mm<n, MM_ACC>(Tm, Y, Rm, Rm);
-      mm<n, MM_SET>(G, T2, X);
-      if (t < n) S.nsm[t] = S.sm[t] + mv_row<n>(Tm, S.wv2, t);
-      team_sync();
-      mm<n, MM_SET>(Tm, X, Y);  // new T- in Y
-      team_sync();
-      // up side: empty (R+ = 0, T+ = I, S+ = 0); down side: (new R-, new T-, new S-)
-      ew_zero<n>(Rp);
-      ew_ident<n>(Tp);
-      for (int ee = t; ee < MAT; ee += T) { R2[ee] = Rm[ee]; T2[ee] = Y[ee]; }
-      if (t < n) { S.sp[t] = 0.0; S.s2m[t] = S.nsm[t]; }
-      team_sync();
-    }
-    // INTERNAL_RADIANCE4 (src/radintg4.f90:119-172): up = (Rp, Tp, sp), down = (R2, T2, s2m)
-    mm<n, MM_SET>(Rp, R2, X);
-    if (t < n) S.wv[t] = mv_row<n>(T2, S.gnd, t);
-    team_sync();
-    double* Ginv;
-    {
-      int sg = 0;
-      Ginv = inv_iminus<n>(X, G, S.inv, &sg);
-      if (sg) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_PIVOT;
-    }
-    if (t < n) {
-      double s = mv_row<n>(Rp, S.wv, t);
-      s = mv_row<n>(Tp, S.sky, t) + s;
-      s = mv_row<n>(Rp, S.s2m, t) + s;
-      s = S.sp[t] + s;
-      S.wv2[t] = s;
-    }
-    team_sync();
-    if (t < n) S.dnrad[t] = mv_row<n>(Ginv, S.wv2, t);
-    team_sync();
-    mm<n, MM_SET>(R2, Rp, X);
-    if (t < n) S.wv[t] = mv_row<n>(Tp, S.sky, t);
-    team_sync();
-    {
-      int sg = 0;
-      Ginv = inv_iminus<n>(X, G, S.inv, &sg);
-      if (sg) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_PIVOT;
-    }
-    if (t < n) {
-      double s = mv_row<n>(R2, S.wv, t);
-      s = mv_row<n>(T2, S.gnd, t) + s;
-      s = mv_row<n>(R2, S.sp, t) + s;
-      s = S.s2m[t] + s;
-      S.wv2[t] = s;
-    }
-    team_sync();
-    if (t < n) S.uprad[t] = mv_row<n>(Ginv, S.wv2, t);
-    team_sync();
-    // collect_output + CONVERT_OUTPUT
-    if (t < N) {
-      const int jj = t;
-      double u0 = S.uprad[2 * jj], u1 = S.uprad[2 * jj + 1], d0 = S.dnrad[2 * jj], d1 = S.dnrad[2 * jj + 1];
-      if (st.outpol_vh) {
-        double iv = 0.5 * (u0 + u1), ih = 0.5 * (u0 - u1);
-        u0 = iv; u1 = ih;
-        iv = 0.5 * (d0 + d1); ih = 0.5 * (d0 - d1);
-        d0 = iv; d1 = ih;
-        u0 = 2.0 * u0; u1 = 2.0 * u1; d0 = 2.0 * d0; d1 = 2.0 * d1;
-      }
-      const int NA = 2 * b.max_nummu;
-      double* tbo = out.tb + ((size_t)c * b.noutlevels + io) * NA * Fm * 2;
-      const size_t up_i = ((size_t)(N - 1 - jj) * Fm + fi) * 2, dn_i = ((size_t)(N + jj) * Fm + fi) * 2;
-      tbo[up_i + 0] = rad_to_tb(u0, wl);
-      tbo[up_i + 1] = rad_to_tb(u1, wl);
-      tbo[dn_i + 0] = rad_to_tb(d0, wl);
-      tbo[dn_i + 1] = rad_to_tb(d1, wl);
-    }
-    team_sync();
-  }
-  if (t == 0) {
-    if (out.emissivity)
-      for (int i = 0; i < 2; i++)
-        for (int jj = 0; jj < N; jj++) out.emissivity[(((size_t)c * 2 + i) * Fm + fi) * b.max_nummu + jj] = e;
-    if (status) atomicOr(&w.status[(size_t)c * Fm + fi], status);
-  }
-}
-
-template <int N, bool ONE_INV = false>
-__global__ void __launch_bounds__(RTCfg<N>::T) k_adding(Batch b, Work w, pamtra_b200_settings st,
-                                                        pamtra_b200_outputs out) {
-  constexpr int n = RTCfg<N>::n, LD = RTCfg<N>::LD, MAT = RTCfg<N>::MAT, T = RTCfg<N>::T;
-  extern __shared__ double smem_raw[];
-  AddSmem<N>& S = *reinterpret_cast<AddSmem<N>*>(smem_raw);
-  const int t = threadIdx.x;
-  const int Lm = b.max_nlyrs, Fm = b.max_nfreq;
-  const int nunits = b.ncol * Fm;
-  if (t < N) { S.mu[t] = w.lob_mu[lob_off(N) + t]; S.wq[t] = w.lob_w[lob_off(N) + t]; }
-  for (;;) {
-    team_sync();
-    if (t == 0) S.unit = atomicAdd(&w.counters[5 + (N == 8 ? 0 : (N == 16 ? 1 : 2))], 1);
-    team_sync();
-    const int unit = S.unit;
-    if (unit >= nunits) break;
-    const int c = unit / Fm, fi = unit % Fm;
-    if (fi >= b.col_nfreq(c) || b.col_nummu(c) != N) continue;
-    const int L = b.nlyrs[c];
-    const double freq = b.freq(c, fi);
-    const double wl = C_LIGHT / (freq * 1.e3);
-    const double* hl = w.hgt_lev + (size_t)c * (Lm + 1);
-    const double* tl = w.temp_lev + (size_t)c * (Lm + 1);
-    int status = w.col_status[c];
-    double* mats[10];
-#pragma unroll
-    for (int q = 0; q < 10; q++)
-      mats[q] = (q < AddSmem<N>::NS) ? S.m[q < AddSmem<N>::NS ? q : 0]
-                                     : w.add_scr + ((size_t)blockIdx.x * (10 - AddSmem<N>::NS) + (q - AddSmem<N>::NS)) * MAT;
-    double *Rp = mats[0], *Rm = mats[1], *Tp = mats[2], *Tm = mats[3];
-    double *R2 = mats[4], *T2 = mats[5];
-    double *G = mats[6], *X = mats[7], *Y = mats[8], *Z = mats[9];
-    // stack state: 0 empty, 1 clear (R = 0, T = diag t1 on both sides), 2 general
-    int sstate = 0;
-    // The next scattering layer's R, T and S blocks are read into registers
-    // while the current combine runs (batched forms, N <= 16: the kernel's
-    // occupancy is set by shared memory, so the registers are free).
-    constexpr bool PREFETCH = ONE_INV && N <= 16;
-    constexpr int PFE = (MAT + T - 1) / T;
-    double pfR[PREFETCH ? PFE : 1], pfT[PREFETCH ? PFE : 1], pfS[2];
-    int pf_pidx = -1;
-    auto prefetch = [&](int kfrom) {
-      pf_pidx = -1;
-      for (int kk = kfrom; kk < L; kk++) {
-        const int p = w.pres_idx[(size_t)c * Lm + (L - 1 - kk)];
-        if (p >= 0) { pf_pidx = p; break; }
-      }
-      if (pf_pidx < 0) return;
-      const double* src = w.lay + ((size_t)pf_pidx * Fm + fi) * w.lay_stride;
-#pragma unroll
-      for (int q = 0; q < PFE; q++) {
-        const int e = t + q * T;
-        if (e < MAT) { pfR[q] = src[e]; pfT[q] = src[MAT + e]; }
-      }
-      if (t < n) { pfS[0] = src[2 * MAT + t]; pfS[1] = src[2 * MAT + n + t]; }
-    };
-    if (PREFETCH) prefetch(0);
-    for (int k = 0; k < L; k++) {  // top-down layer index
-      const int z = L - 1 - k;
-      const int pidx = w.pres_idx[(size_t)c * Lm + z];
-      if (pidx < 0) {
-        // NONSCATTER_LAYER4 (src/radintg4.f90:79-117)
-        if (t < n) {
-          const int jj = t >> 1, i = t & 1;
-          const double zdiff = fabs(hl[z + 1] - hl[z]);
-          const double gas = fmax(w.kgas[((size_t)c * Fm + fi) * Lm + z], 0.0);
-          const double dtau = zdiff * gas;
-          const double p0 = planck(tl[z + 1], wl), p1 = planck(tl[z], wl);
-          S.t2[t] = exp(-dtau / S.mu[jj]);
-          double a = 0.0, bq = 0.0;
-          if (dtau > 0.0 && i == 0) {
-            const double path = dtau / S.mu[jj];
-            const double slope = (p1 - p0) / path;
-            a = p1 - slope - (p1 - slope * (1.0 + path)) * exp(-path);
-            bq = p0 + slope - (p0 + slope * (1.0 + path)) * exp(-path);
-          }
-          S.s2p[t] = a;
-          S.s2m[t] = bq;
-        }
-        team_sync();
-        if (sstate == 0) {
-          if (t < n) { S.t1[t] = S.t2[t]; S.sp[t] = S.s2p[t]; S.sm[t] = S.s2m[t]; }
-          sstate = 1;
-        } else if (sstate == 1) {
-          // clear + clear
-          if (t < n) {
-            const double sp = S.s2p[t] + S.t2[t] * S.sp[t];
-            const double sm = S.sm[t] + S.t1[t] * S.s2m[t];
-            S.t1[t] = S.t2[t] * S.t1[t];
-            S.sp[t] = sp;
-            S.sm[t] = sm;
-          }
-        } else {
-          // general stack + clear layer
-          if (t < n) S.nsp[t] = S.s2p[t] + S.t2[t] * (S.sp[t] + mv_row<n>(Rp, S.s2m, t));
-          else if (t < 2 * n) S.nsm[t - n] = S.sm[t - n] + mv_row<n>(Tm, S.s2m, t - n);
-          team_sync();
-          for (int e = t; e < n * n; e += T) {
-            const int col = e / n, row = e % n, a = col * LD + row;
-            const double t2i = S.t2[row], t2j = S.t2[col];
-            Rp[a] = t2i * (Rp[a] * t2j);
-            Tp[a] = t2i * Tp[a];
-            Tm[a] = Tm[a] * t2j;
-          }
-          if (t < n) { S.sp[t] = S.nsp[t]; S.sm[t] = S.nsm[t]; }
-        }
-        team_sync();
-        continue;
-      }
-      // scattering layer: its R2, T2, S2 from the arena (prefetched), then the next one's
-      if (PREFETCH) {
-#pragma unroll
-        for (int q = 0; q < PFE; q++) {
-          const int e = t + q * T;
-          if (e < MAT) { R2[e] = pfR[q]; T2[e] = pfT[q]; }
-        }
-        if (t < n) { S.s2p[t] = pfS[0]; S.s2m[t] = pfS[1]; }
-        prefetch(k + 1);
-      } else {
-        const double* src = w.lay + ((size_t)pidx * Fm + fi) * w.lay_stride;
-        for (int e = t; e < MAT; e += T) { R2[e] = src[e]; T2[e] = src[MAT + e]; }
-        for (int e = t; e < n; e += T) { S.s2p[e] = src[2 * MAT + e]; S.s2m[e] = src[2 * MAT + n + e]; }
-      }
-      team_sync();
-      if (sstate == 0) {
-        for (int e = t; e < MAT; e += T) { Rp[e] = R2[e]; Rm[e] = R2[e]; Tp[e] = T2[e]; Tm[e] = T2[e]; }
-        if (t < n) { S.sp[t] = S.s2p[t]; S.sm[t] = S.s2m[t]; }
-        sstate = 2;
-        team_sync();
-        continue;
-      }
-      if (sstate == 1) {
-        // clear stack (t1, sp, sm) + scattering layer
-        if (t < n) S.nsp[t] = S.s2p[t] + mv_row<n>(T2, S.sp, t);
-        else if (t < 2 * n) S.nsm[t - n] = S.sm[t - n] + S.t1[t - n] * (S.s2m[t - n] + mv_row<n>(R2, S.sp, t - n));
-        for (int e = t; e < n * n; e += T) {
-          const int col = e / n, row = e % n, a = col * LD + row;
-          const double t1i = S.t1[row], t1j = S.t1[col];
-          const double r2 = R2[a], tt = T2[a];
-          Rp[a] = r2;
-          Rm[a] = t1i * (r2 * t1j);
-          Tp[a] = tt * t1j;
-          Tm[a] = t1i * tt;
-        }
-        team_sync();
-        if (t < n) { S.sp[t] = S.nsp[t]; S.sm[t] = S.nsm[t]; }
-        sstate = 2;
-        team_sync();
-        continue;
-      }
-      if (ONE_INV) {
-        // ---- COMBINE_LAYERS4 with one inverse.  With Gp = (I - R1p R2)^-1
-        // the minus-side inverse Gm = (I - R2 R1p)^-1 satisfies
-        //   Gm R2 = R2 Gp   and   Gm = I + R2 Gp R1p,
-        // so R1m' = R1m + T1m Gm R2 T1p = R1m + (T1m R2)(Gp T1p),
-        //    T1m' = T1m Gm T2 = T1m (T2 + R2 (Gp R1p T2)),
-        //    Gm w = w + R2 Gp (R1p w) for the S- chain:
-        // ten products and one inverse per combine instead of twelve and two.
-        // Products that share their left factor run in one pass (mm2), and the
-        // two source chains of a phase run on different warps:
-        //   Rp [R2, T2] -> Gp (inverted next), Z = R1p T2
-        mm2<n, MM_SET, MM_SET>(Rp, R2, G, nullptr, T2, Z, nullptr);
-        if (t < n) S.wv[t] = S.sp[t] + mv_row<n>(Rp, S.s2m, t);                    // S+ chain
-        else if (t < 2 * n) S.nsm[t - n] = S.s2m[t - n] + mv_row<n>(R2, S.sp, t - n);  // S- chain: w
-        team_sync();
-        {
-          int sg = 0;
-          double* gi = inv_iminus<n>(G, X, S.inv, &sg);
-          if (sg) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_PIVOT;
-          if (gi != G) { X = G; G = gi; }
-        }
-        //   Gp [Z, T1p] -> Y = Gp R1p T2, X = W = Gp T1p
-        mm2<n, MM_SET, MM_SET>(G, Z, Y, nullptr, Tp, X, nullptr);
-        if (t < n) S.wv2[t] = mv_row<n>(G, S.wv, t);
-        else if (t < 2 * n) S.u1[t - n] = mv_row<n>(Rp, S.nsm, t - n);
-        team_sync();
-        //   T2 [Y, W] -> new R+ = R2 + T2 Y (into Z), new T+ = T2 W (into Rp: old R+ is dead)
-        mm2<n, MM_ACC, MM_SET>(T2, Y, Z, R2, X, Rp, nullptr);
-        if (t < n) S.nsp[t] = S.s2p[t] + mv_row<n>(T2, S.wv2, t);
-        else if (t < 2 * n) S.u2[t - n] = mv_row<n>(G, S.u1, t - n);
-        team_sync();
-        mm<n, MM_SET>(Tm, R2, G);  // V = T1m R2 (Gp is dead)
-        if (t < n) S.u1[t] = S.nsm[t] + mv_row<n>(R2, S.u2, t);  // Gm w
-        team_sync();
-        mm<n, MM_ACC>(G, X, Rm, Rm);   // new R- = R1m + V W
-        mm<n, MM_ACC>(R2, Y, Tp, T2);  // U = T2 + R2 Y (old T+ is dead)
-        if (t < n) S.nsm[t] = S.sm[t] + mv_row<n>(Tm, S.u1, t);
-        team_sync();
-        mm<n, MM_SET>(Tm, Tp, X);  // new T- = T1m U
-        team_sync();
-        {
-          // roles: new R+ = Z, new R- = Rm, new T+ = Rp, new T- = X
-          double *oRp = Rp, *oTp = Tp, *oTm = Tm, *oX = X, *oZ = Z;
-          Rp = oZ;
-          Tp = oRp;
-          Tm = oX;
-          Z = oTp;
-          X = oTm;
-        }
-        if (t < n) { S.sp[t] = S.nsp[t]; S.sm[t] = S.nsm[t]; }
-        team_sync();
-        continue;
-      }
-      // ---- general COMBINE_LAYERS4 (src/radintg4.f90:447-513), R2p = R2m, T2p = T2m
-      mm<n, MM_SET>(Rp, R2, G);  // GAMMAp = inv(I - R1p R2m)
-      team_sync();
-      {
-        int sg = 0;
-        double* gi = inv_iminus<n>(G, X, S.inv, &sg);
-        if (sg) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_PIVOT;
-        if (gi != G) { X = G; G = gi; }
-      }
-      mm<n, MM_SET>(Rp, T2, X);  // RTp = R2p + T2p G R1p T2m
-      if (t < n) S.wv[t] = S.sp[t] + mv_row<n>(Rp, S.s2m, t);  // STp chain
-      team_sync();
-      mm<n, MM_SET>(G, X, Y);
-      if (t < n) S.wv2[t] = mv_row<n>(G, S.wv, t);
-      team_sync();
-      mm<n, MM_ACC>(T2, Y, Z, R2);  // new R+ in Z
-      mm<n, MM_SET>(G, Tp, X);      // TTp = T2p G T1p
-      if (t < n) S.nsp[t] = S.s2p[t] + mv_row<n>(T2, S.wv2, t);
-      team_sync();
-      mm<n, MM_SET>(T2, X, Y);  // new T+ in Y
-      team_sync();
-      mm<n, MM_SET>(R2, Rp, G);  // GAMMAm = inv(I - R2m R1p); Gp is dead
-      team_sync();
-      {
-        int sg = 0;
-        double* gi = inv_iminus<n>(G, X, S.inv, &sg);
-        if (sg) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_PIVOT;
-        if (gi != G) { X = G; G = gi; }
-      }
-      mm<n, MM_SET>(R2, Tp, X);  // RTm = R1m + T1m G R2m T1p
-      if (t < n) S.wv[t] = S.s2m[t] + mv_row<n>(R2, S.sp, t);  // STm chain
-      team_sync();
-      mm<n, MM_SET>(G, X, Rp);  // old R+ is dead
-      if (t < n) S.wv2[t] = mv_row<n>(G, S.wv, t);
-      team_sync();
-      mm<n, MM_ACC>(Tm, Rp, Rm, Rm);  // new R- in place
-      mm<n, MM_SET>(G, T2, X);        // TTm = T1m G T2m
-      if (t < n) S.nsm[t] = S.sm[t] + mv_row<n>(Tm, S.wv2, t);
-      team_sync();
-      mm<n, MM_SET>(Tm, X, Tp);  // old T+ is dead: new T- in Tp buffer
-      team_sync();
-      {
-        // roles: new R+ = Z, new R- = Rm, new T+ = Y, new T- = Tp
-        double *oRp = Rp, *oTm = Tm;
-        Rp = Z;
-        Tm = Tp;
-        Tp = Y;
-        Z = oRp;
-        Y = oTm;
-      }
-      if (t < n) { S.sp[t] = S.nsp[t]; S.sm[t] = S.nsm[t]; }
-      team_sync();
-    }
-    adding_finish<N>(b, w, st, out, S, c, fi, L, wl, sstate, status, Rp, Rm, Tp, Tm, R2, T2, G, X, Y);
   }
 }
 

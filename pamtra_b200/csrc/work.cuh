@@ -70,14 +70,14 @@ struct Work {
   int mie_nslab;
   double* m_legen;                     // [pmax*Fm][3][MAXNLEG] normalised Legendre coefficients (FP64 storage)
   float* m_legen32;                    // the same in FP32 storage (split-precision form); exactly one is set
-  // layer R, T, S per item (R,T padded n x (n+2), symmetric +/-)
+  // layer R, T, S+, S- per item: scaled and swizzled (k_layer), or n x (n + 4) unscaled
+  // (split-precision doubling), or FP32 (lay32).  k_adding keeps its segments' stacks here
   double* lay;                         // [pmax*Fm][lay_stride]
   size_t lay_stride;
   int* lay_nd;                         // [pmax*Fm]
   int lay32;                           // k_layer_tc writes FP32 layer records (add_tc.cuh) for k_adding_tc
   float* add_stk;                      // [C*Fm][STK_FLOATS] FP32 adding stacks, k_adding_tc -> k_adding_finish
-  // adding matrices that do not fit in shared memory (N = 32 only)
-  double* add_scr;                     // [adding CTAs][4][MAT]
+  int* seg_cnt;                        // [C*Fm] segments of the unit k_adding has finished (zero at the start)
   // scatcnv weight tables per NUMMU index (0: N = 8, 1: 16, 2: 32); null = direct sums
   const double* wtab[3];               // [numpts index][l][5][2 N^2], see scat_weight_offset
   int* wt_need;                        // [3][SCAT_NPI] numpts values seen (set by k_mie)

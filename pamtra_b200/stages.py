@@ -2,8 +2,8 @@
 
 ``python -m pamtra_b200.stages [--workload c2|target|uneven|mieheavy] [--ncol N]
 [--precision fp64|fp64b|3xtf32|3xtf32d|both|all] [--reps K]`` runs one untimed and
-K timed batches per precision (fp64: the reference operation order, fp64b:
-the batched FP64 form, 3xtf32: the split-precision form, 3xtf32d: its
+K timed batches per precision (fp64: FP64, fp64b:
+the batched FP64 form, which runs the same kernels, 3xtf32: the split-precision form, 3xtf32d: its
 doubling with the FP64 adding) through
 :func:`pamtra_b200.batch.run` and prints one JSON line per precision:
 milliseconds per stage (CUDA events the library records between its kernels
