@@ -581,6 +581,7 @@ def _tmatrix_line(args, eng, dev, cpu_leg, pool=None, cores=1):
         return e0.elapsed_time(e1) / steps, o, a
 
     ms, o, a = timed(ni, 0.0, 3)
+    launches = eng.last_launch_count()
     nm = o["nmax"].cpu().numpy()
     # e2e: numpy arrays through the host path of the C-ABI (copies in the call)
     h = arrays(ni, 0.0)
@@ -602,11 +603,11 @@ def _tmatrix_line(args, eng, dev, cpu_leg, pool=None, cores=1):
             "nmax_range": [int(nm.min()), int(nm.max())], "status_nonzero": int(np.count_nonzero(o["status"].cpu().numpy())),
             "e2e": {"value": ni * nb / e2e_s, "unit": "bins/s", "h2d_bytes_per_step": int(h2d),
                     "d2h_bytes_per_step": int(d2h)},
-            "gpu_launches_per_step": 3,
+            "gpu_launches_per_step": launches,
             "canted": {"value": nc * nb / (ms_c * 1e-3), "unit": "bins/s", "items": nc, "beta_deg": 20.0,
-                       "form": "full AMPL per (incident angle, scattered angle, azimuth)"},
-            "bound": "latency: one FP64 CTA chain per bin (solves of order 2 (NMAX - m + 1) with a CTA barrier "
-                     "per pivot, then the angular sums); no tensor-core or HBM bound applies"}
+                       "form": "P_m per scattered direction, summed over m per incident angle"},
+            "bound": "latency: an FP64 chain per bin (convergence steps and pivots one after another, solves of a "
+                     "bin side by side), then the angular sums; no tensor-core or HBM bound applies"}
     if cpu_leg:
         sys.path.insert(0, os.path.join(ROOT, "oracle"))
         import oracle

@@ -464,6 +464,7 @@ struct pamtra_b200_ctx {
   double* wtab[3] = {nullptr, nullptr, nullptr};
   int* wt_flags = nullptr;
   int last_launches = 0;
+  double* tm_tab = nullptr;  // T-matrix branch: tables (TMT_*), then the directions of upright particles per nummu
   char* tm_buf = nullptr;  // T-matrix branch: inputs, per-bin results and the CTAs' scratch slots
   size_t tm_bytes = 0;
   char* stage = nullptr;  // device staging for run_host
@@ -528,8 +529,14 @@ static int set_smem_attrs() {
     set((const void*)k_minvert<64>, Team<64>::MAT * 8 + sizeof(InvScratch<64>));
     set((const void*)k_adding_tc<16>, add_tc_smem());
     set((const void*)k_adding_finish<16>, sizeof(AddSmem<16>));
+    set((const void*)k_tmat_ampl, TMA_SMEM * 8);
   });
   return rc;
+}
+
+// the directions table of one nummu (8, 16 or 32)
+static double* tm_geo_of(double* tab, int nummu) {
+  return tab + TMT_TOTAL + (nummu > 8 ? tm_geo_doubles(8) : 0) + (nummu > 16 ? tm_geo_doubles(16) : 0);
 }
 
 extern "C" {
@@ -561,6 +568,14 @@ int32_t pamtra_b200_create(int32_t device, pamtra_b200_ctx** out) {
   }
   upload_mie_constants();
   k_lobatto_table<<<3, 32>>>(ctx->lob_mu, ctx->lob_w);
+  if (cudaMalloc(&ctx->tm_tab, (TMT_TOTAL + tm_geo_doubles(8) + tm_geo_doubles(16) + tm_geo_doubles(32)) * 8)) {
+    delete ctx;
+    return PAMTRA_B200_FATAL;
+  }
+  k_tmat_tables<<<TM_NGAUSS + 1, TM_NGAUSS>>>(ctx->tm_tab);
+  for (int nummu = 8; nummu <= 32; nummu *= 2)
+    k_tmat_geo<<<(2 * nummu * TM_NAZ + nummu + 127) / 128, 128>>>(tm_geo_of(ctx->tm_tab, nummu), nummu, ctx->lob_mu + lob_off(nummu));
+  k_tmat_azimuth<<<1, 32>>>(ctx->tm_tab, tm_geo_of(ctx->tm_tab, 8), 8);
   cudaMemcpyToSymbol(c_o2_w300, H_O2_W300, sizeof(H_O2_W300));
   cudaMemcpyToSymbol(c_o2_y300, H_O2_Y300, sizeof(H_O2_Y300));
   cudaMemcpyToSymbol(c_o2_v, H_O2_V, sizeof(H_O2_V));
@@ -592,6 +607,7 @@ int32_t pamtra_b200_destroy(pamtra_b200_ctx* ctx) {
   cudaFree(ctx->lob_w);
   cudaFree(ctx->stage);
   cudaFree(ctx->tm_buf);
+  cudaFree(ctx->tm_tab);
   for (double* p : ctx->wtab) cudaFree(p);
   cudaFree(ctx->wt_flags);
   for (auto& sg : ctx->sp_ring) {
@@ -1225,8 +1241,15 @@ int32_t pamtra_b200_tmatrix(pamtra_b200_ctx* ctx, const pamtra_b200_tmatrix_in* 
   cudaStream_t stream = (cudaStream_t)stream_;
   const size_t n = (size_t)ni * nb;
   const size_t NS = (size_t)2 * nummu * 2 * nummu * 2, NE = 4 * (size_t)nummu, NM = 2 * (size_t)nummu;
-  // two 256-thread CTAs per SM (128 registers per thread), persistent
+  // sixteen warps per SM (128 registers per thread): two persistent CTAs
   const int grid = (int)std::min<size_t>(n, (size_t)2 * ctx->sm_count);
+  const int agrid = 3 * ctx->sm_count;
+  // records of the particles: room for all of them up to TM_RECORD_BYTES, then
+  // rounds; a round holds at least rec / rmax - 1 particles of the largest order
+  constexpr size_t TM_RECORD_BYTES = (size_t)1 << 30;
+  const size_t rmax = std::max(tm_record(TM_PAIRS, nummu, true), tm_record(TM_PAIRS, nummu, false));
+  const size_t rec = std::min(n * rmax, TM_RECORD_BYTES / 8);
+  const int rounds = n * rmax <= rec ? 1 : (int)((n + rec / rmax - 2) / (rec / rmax - 1));
   // device layout (8-byte units, each array 256-byte aligned)
   size_t off = 0;
   auto take = [&](size_t elems8) { const size_t o = off; off += (elems8 + 31) / 32 * 32; return o; };
@@ -1235,10 +1258,14 @@ int32_t pamtra_b200_tmatrix(pamtra_b200_ctx* ctx, const pamtra_b200_tmatrix_in* 
   const size_t o_dmax = take(n), o_dd = take(n), o_nd = take(n), o_rho = take(n), o_asr = take(n), o_cant = take(n);
   const size_t o_mrr = take(n), o_mri = take(n), o_axi = take(n), o_nde = take(n), o_pst = take((n + 1) / 2),
                o_pnm = take((n + 1) / 2);
-  const size_t o_pscat = take(n * NS), o_pext = take(n * NE), o_pemis = take(n * NM), o_psb = take(n * 4);
+  const size_t o_pscat = take(n * NS), o_pext = take(n * NE), o_psb = take(n * 4);
   const size_t o_scat = take((size_t)ni * NS), o_ext = take((size_t)ni * NE), o_emis = take((size_t)ni * NM),
-               o_sb = take((size_t)ni * 4), o_back = take(n), o_st = take(((size_t)ni + 1) / 2), o_cnt = take(1);
-  const size_t o_slot = take((size_t)grid * TM_SLOT_DOUBLES);
+               o_sb = take((size_t)ni * 4), o_back = take(n), o_st = take(((size_t)ni + 1) / 2);
+  const size_t o_key = take((n + 1) / 2), o_ord0 = take((n + 1) / 2), o_ord1 = take((n + 1) / 2),
+               o_upr = take((n + 1) / 2), o_cnt = take((n + 1) / 2), o_rec = take(n);
+  const size_t o_rounds = take(((size_t)rounds + 1) * sizeof(TmRound) / 8);
+  const size_t o_slot = take((size_t)grid * tm_slot(nummu).total), o_aslot = take((size_t)agrid * TMA_SLOT);
+  const size_t o_records = take(rec);
   const size_t bytes = off * 8;
   if (bytes > ctx->tm_bytes) {
     cudaStreamSynchronize(stream);
@@ -1263,25 +1290,38 @@ int32_t pamtra_b200_tmatrix(pamtra_b200_ctx* ctx, const pamtra_b200_tmatrix_in* 
     dmax = D(o_dmax); dd = D(o_dd); nd = D(o_nd); rho = D(o_rho); asr = D(o_asr); cant = D(o_cant);
   }
   k_tmat_prep<<<(unsigned)((n + 127) / 128), 128, 0, stream>>>(ni, nb, freq, rre, rim, phase, dmax, dd, nd, rho, asr, cant,
-                                                                D(o_mrr), D(o_mri), D(o_axi), D(o_nde), I(o_pst));
-  cudaMemsetAsync(I(o_cnt), 0, 4, stream);
+                                                                D(o_mrr), D(o_mri), D(o_axi), D(o_nde), I(o_pst), I(o_key));
+  TmRound* rd = reinterpret_cast<TmRound*>(B + o_rounds * 8);
+  cudaMemsetAsync(rd, 0, ((size_t)rounds + 1) * sizeof(TmRound), stream);
+  k_tmat_order<<<1, 1024, 0, stream>>>((int)n, I(o_key), I(o_ord0), rd);
   TmArgs A;
   A.n_items = ni; A.nbins = nb; A.nummu = nummu;
   A.freq = freq; A.mrr = D(o_mrr); A.mri = D(o_mri); A.axi = D(o_axi); A.asr = asr; A.beta = cant; A.ndens = D(o_nde);
+  A.tab = ctx->tm_tab; A.geo = tm_geo_of(ctx->tm_tab, nummu);
   A.mu = ctx->lob_mu + lob_off(nummu); A.wq = ctx->lob_w + lob_off(nummu);
-  A.scat = D(o_pscat); A.ext = D(o_pext); A.emis = D(o_pemis); A.sback = D(o_psb);
+  A.scat = D(o_pscat); A.ext = D(o_pext); A.sback = D(o_psb);
   A.nmax = (!host && out->nmax) ? out->nmax : I(o_pnm);
-  A.status = I(o_pst); A.scratch = D(o_slot); A.counter = I(o_cnt);
-  k_tmatrix<<<grid, TM_THREADS, 0, stream>>>(A);
+  A.status = I(o_pst); A.scratch = D(o_slot); A.ascratch = D(o_aslot);
+  A.records = D(o_records); A.rec_doubles = rec; A.rec = reinterpret_cast<int64_t*>(B + o_rec * 8);
+  A.upright = I(o_upr); A.canted = I(o_cnt);
+  for (int r = 0; r < rounds; r++) {
+    A.order = I(r & 1 ? o_ord1 : o_ord0);
+    A.again = I(r & 1 ? o_ord0 : o_ord1);
+    A.round = rd + r;
+    A.next = rd + r + 1;
+    k_tmatrix<<<grid, TM_THREADS, 0, stream>>>(A);
+    k_tmat_ampl<<<agrid, TMA_THREADS, TMA_SMEM * 8, stream>>>(A);
+  }
   double *scat = out->scatter_matrix, *ext = out->extinct_matrix, *emis = out->emis_vector, *sb = out->sback,
          *back = out->back_spec;
   int* st = out->status;
   if (host) {
     scat = D(o_scat); ext = D(o_ext); emis = D(o_emis); sb = D(o_sb); back = D(o_back); st = I(o_st);
   }
-  k_tmat_sum<<<ni, 256, 0, stream>>>(ni, nb, nummu, D(o_nde), dd, D(o_pscat), D(o_pext), D(o_pemis), D(o_psb), I(o_pst),
-                                     scat, ext, emis, sb, back, st);
-  ctx->last_launches = 3;
+  k_tmat_sum<<<dim3(ni, (unsigned)((NS + NE + 4 + 255) / 256)), 256, 0, stream>>>(
+      ni, nb, nummu, D(o_nde), dd, D(o_pscat), D(o_pext), D(o_psb), I(o_pst), scat, ext, sb, back, st);
+  k_tmat_emis<<<(unsigned)((ni * NM + 127) / 128), 128, 0, stream>>>(ni, nummu, A.wq, scat, ext, emis);
+  ctx->last_launches = 4 + 2 * rounds;
   if (cudaGetLastError() != cudaSuccess) return PAMTRA_B200_FATAL;
   if (host) {
     auto dn = [&](void* dst, size_t o, size_t b) { cudaMemcpyAsync(dst, B + o * 8, b, cudaMemcpyDeviceToHost, stream); };

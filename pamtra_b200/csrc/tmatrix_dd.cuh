@@ -46,7 +46,8 @@ __device__ bool tdd_setup(double* sd, TmShared& sh, int nmax, int ngauss, double
 }
 
 // TMATR0 / TMATR + TT (tmatrix_amplq.lp.f:1526-2153) in double-double for
-// order m; T goes where tm_tget of the FP64 slot s reads it.  Whole CTA;
+// order m; T^T goes to the right half of one [2 nm][4 nm] array at the start of
+// the slot s (the FP64 solve keeps an array per decoupled system).  Whole CTA;
 // returns 2 nm, or 0 when a pivot vanishes.
 __device__ int tdd_solve(double* s, double* sd, TmShared& sh, int m, int nmax, int ngauss, double lam, double mrr,
                          double mri) {
