@@ -219,8 +219,9 @@ int32_t pamtra_b200_run_host(pamtra_b200_ctx* ctx, const pamtra_b200_settings* s
  * autotuner (pamtra_b200/autotune.py); no counterpart in the reference, whose
  * Fortran has no launch configuration.  params[0]: warps per Mie CTA (2, 4 or
  * 8; 0 = 4), params[1..3]: CTAs per SM of the Mie, layer and adding kernels
- * (0 = as many as fit), params[4]: size bins per Mie work item, the tile of
- * the phase-function sums (4 or 8; 0 = 4).  Results do not depend on the
+ * (0 = as many as fit), params[4]: the tile of the
+ * Mie phase-function sums, eight angles and their mirror images (4) or sixteen
+ * (8; 0 = 4).  Results do not depend on the
  * launch shape. */
 #define PAMTRA_B200_NLAUNCH 5
 int32_t pamtra_b200_set_launch(pamtra_b200_ctx* ctx, const int32_t* params, int32_t n);
@@ -360,8 +361,8 @@ int32_t pamtra_b200_mmult_3xtf32_batched(const double* a, const double* b, doubl
  * callers that cannot accept the device-wide synchronisation an allocation
  * implies.  Runs the plain form (one column, same kernels as
  * pamtra_b200_run) with all scratch in a fixed static device array of
- * PAMTRA_B200_NOALLOC_SCRATCH_MIB MiB that every GPU loading this library
- * keeps until the process exits.  No context is needed and nothing is
+ * PAMTRA_B200_NOALLOC_SCRATCH_MIB MiB (and 21 MiB of Mie tables) that every
+ * GPU loading this library keeps until the process exits.  No context is needed and nothing is
  * allocated: no cudaMalloc, cudaFree, pinned host memory or library
  * allocator.  All pointers in `cols` and `out` are DEVICE pointers,
  * `cols->species` included.  Limits: ncol = 1, max_nlyrs <= 64,

@@ -8,8 +8,8 @@ species) the tuner times candidate shapes with the library's per-stage CUDA
 events and keeps, stage by stage, the fastest:
 
 * Mie: warps per CTA (2, 4, 8), CTAs per SM, and the tile of its
-  phase-function sums (size bins per work item: 4 or 8, two compiled
-  instantiations of the kernel),
+  phase-function sums (4: eight angles and their mirror images, 8: sixteen;
+  two compiled instantiations of the kernel),
 * layer doubling: CTAs per SM (FP64 teams, or item pairs of the
   split-precision kernel),
 * adding: CTAs per SM,
@@ -32,8 +32,8 @@ import numpy as np
 
 from ._native import PREC_FP64, engine
 
-# candidate rows: (mie warps, mie CTAs/SM, layer CTAs/SM, adding CTAs/SM, mie bins per work
-# item); 0 = as many as fit (CTAs) or the default (warps, bins)
+# candidate rows: (mie warps, mie CTAs/SM, layer CTAs/SM, adding CTAs/SM, mie angle tile);
+# 0 = as many as fit (CTAs) or the default (warps, tile)
 CANDIDATES = [
     (4, 0, 0, 0, 4),
     (8, 0, 1, 1, 8),

@@ -445,6 +445,7 @@ struct pamtra_b200_ctx {
   size_t arena_bytes = 0;
   double* gq_x = nullptr;
   double* gq_w = nullptr;
+  double* mie_tab = nullptr;  // angular tables of k_mie
   double* lob_mu = nullptr;
   double* lob_w = nullptr;
   // species tables: pinned staging ring and the table last left in the arena
@@ -474,7 +475,7 @@ struct pamtra_b200_ctx {
   int mie_cps = 0;            // k_mie CTAs per SM
   int layer_cps = 0;          // k_layer / k_layer_tc CTAs per SM
   int adding_cps = 0;         // k_adding CTAs per SM
-  int mie_group = MIE_GROUP;  // bins per k_mie work item (4 or 8)
+  int mie_group = 4;  // k_mie angle tiles per item: one pair (4) or two (8)
   uint32_t spin_limit = tc::MBAR_SPIN_LIMIT;  // polls per wait on a tensor-core MMA
   const int* last_counters = nullptr;          // work counters of the last run (in the arena)
   // optional per-stage timing (events recorded on the run's stream)
@@ -503,8 +504,12 @@ static int upload_mie_constants() {
   r[0] = 0.0;
   for (int n = 1; n <= NT_MAX; n++) c[n] = (double)((float)(2 * n + 1) / (float)(n * (n + 1)));
   for (int n = 1; n < MAXNLEG; n++) r[n] = 1.0 / n;
+  int off[2][NT_MAX] = {}, o = 0;  // all c_n (pi_n +- tau_n) tables, then all P_l ones
+  for (int nt = 1; nt < NT_MAX; o += mie_ptab(nt++)) off[0][nt] = o;
+  for (int nt = 1; nt < NT_MAX; o += mie_ltab(nt++)) off[1][nt] = o;
   return (cudaMemcpyToSymbol(c_mie_c, c, sizeof(c)) != cudaSuccess ||
-          cudaMemcpyToSymbol(c_mie_inv, r, sizeof(r)) != cudaSuccess) ? 1 : 0;
+          cudaMemcpyToSymbol(c_mie_inv, r, sizeof(r)) != cudaSuccess ||
+          cudaMemcpyToSymbol(c_mie_toff, off, sizeof(off)) != cudaSuccess) ? 1 : 0;
 }
 
 static int set_smem_attrs() {
@@ -514,8 +519,8 @@ static int set_smem_attrs() {
     auto set = [](const void* f, size_t bytes) {
       if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) != cudaSuccess) rc = 1;
     };
-    set((const void*)k_mie<4>, MIE_MAX_WARPS * sizeof(MieSmem));
-    set((const void*)k_mie<8>, MIE_MAX_WARPS * sizeof(MieSmem));
+    set((const void*)k_mie<1>, MIE_MAX_WARPS * sizeof(MieSmem));
+    set((const void*)k_mie<2>, MIE_MAX_WARPS * sizeof(MieSmem));
     set((const void*)k_layer<8>, sizeof(LayerSmem<8>));
     set((const void*)k_layer<16>, sizeof(LayerSmem<16>));
     set((const void*)k_layer<32>, sizeof(LayerSmem<32>));
@@ -549,7 +554,7 @@ int32_t pamtra_b200_create(int32_t device, pamtra_b200_ctx** out) {
   cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device);
   if (set_smem_attrs()) { delete ctx; return PAMTRA_B200_FATAL; }
   const size_t gq_n = (size_t)GQ_MAX * (GQ_MAX + 1) / 2;
-  if (cudaMalloc(&ctx->gq_x, gq_n * 8) || cudaMalloc(&ctx->gq_w, gq_n * 8) || cudaMalloc(&ctx->lob_mu, 56 * 8) ||
+  if (cudaMalloc(&ctx->gq_x, gq_n * 8) || cudaMalloc(&ctx->gq_w, gq_n * 8) || cudaMalloc(&ctx->mie_tab, MIE_TAB * 8) || cudaMalloc(&ctx->lob_mu, 56 * 8) ||
       cudaMalloc(&ctx->lob_w, 56 * 8)) {
     delete ctx;
     return PAMTRA_B200_FATAL;
@@ -567,6 +572,7 @@ int32_t pamtra_b200_create(int32_t device, pamtra_b200_ctx** out) {
     cudaMemcpyToSymbol(c_leg_b, lb, sizeof(lb));
   }
   upload_mie_constants();
+  k_mie_tables<<<NT_MAX - 1, 128>>>(ctx->mie_tab, ctx->gq_x);
   k_lobatto_table<<<3, 32>>>(ctx->lob_mu, ctx->lob_w);
   if (cudaMalloc(&ctx->tm_tab, (TMT_TOTAL + tm_geo_doubles(8) + tm_geo_doubles(16) + tm_geo_doubles(32)) * 8)) {
     delete ctx;
@@ -603,6 +609,7 @@ int32_t pamtra_b200_destroy(pamtra_b200_ctx* ctx) {
   cudaFree(ctx->arena);
   cudaFree(ctx->gq_x);
   cudaFree(ctx->gq_w);
+  cudaFree(ctx->mie_tab);
   cudaFree(ctx->lob_mu);
   cudaFree(ctx->lob_w);
   cudaFree(ctx->stage);
@@ -732,7 +739,7 @@ int32_t pamtra_b200_set_launch(pamtra_b200_ctx* ctx, const int32_t* params, int3
   ctx->mie_cps = v[1];
   ctx->layer_cps = v[2];
   ctx->adding_cps = v[3];
-  ctx->mie_group = v[4] ? v[4] : MIE_GROUP;
+  ctx->mie_group = v[4] ? v[4] : 4;
   return PAMTRA_B200_OK;
 }
 
@@ -905,7 +912,7 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   for (int i = 0; i < 3; i++) w.wtab[i] = ctx->wt_flags ? ctx->wtab[i] : nullptr;
   w.wt_need = ctx->wt_flags;
   w.wt_ready = ctx->wt_flags ? ctx->wt_flags + 3 * SCAT_NPI : nullptr;
-  w.gq_x = ctx->gq_x; w.gq_w = ctx->gq_w; w.gq_max = GQ_MAX; w.lob_mu = ctx->lob_mu; w.lob_w = ctx->lob_w;
+  w.gq_x = ctx->gq_x; w.gq_w = ctx->gq_w; w.gq_max = GQ_MAX; w.mie_tab = ctx->mie_tab; w.lob_mu = ctx->lob_mu; w.lob_w = ctx->lob_w;
 
   int launches = 0;
   ctx->nev = 0;
@@ -943,12 +950,12 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   if (H > 0) {
     const int mw = ctx->mie_warps;
     const size_t sm_mie = mw * sizeof(MieSmem);
-    const void* kmie = ctx->mie_group == 8 ? (const void*)k_mie<8> : (const void*)k_mie<4>;
+    const void* kmie = ctx->mie_group == 8 ? (const void*)k_mie<2> : (const void*)k_mie<1>;
     int g = std::min(persistent_grid(kmie, 32 * mw, sm_mie, sms, ctx->mie_cps), std::max(1, pl.mie_nslab / mw));
     const size_t nref = (size_t)std::max(1, pl.pmax) * Fm;
     k_refr<<<(unsigned)((nref + 127) / 128), 128, 0, stream>>>(b, w, *st); launches++;
-    if (ctx->mie_group == 8) k_mie<8><<<g, 32 * mw, sm_mie, stream>>>(b, w, *st);
-    else k_mie<4><<<g, 32 * mw, sm_mie, stream>>>(b, w, *st);
+    if (ctx->mie_group == 8) k_mie<2><<<g, 32 * mw, sm_mie, stream>>>(b, w, *st);
+    else k_mie<1><<<g, 32 * mw, sm_mie, stream>>>(b, w, *st);
     launches++;
     if (w.wtab[0] && (mask & 1)) {
       k_scat_weights<8><<<SCAT_NPI * ((2 * 8 * 8 + 127) / 128), 128, 0, stream>>>(ctx->wtab[0], w.wt_need, w.wt_ready, ctx->lob_mu);
@@ -1375,12 +1382,14 @@ constexpr int NOALLOC_GQ = 256;
 // k_mie warps of the allocation-free path (each takes a coefficient slab of the scratch)
 constexpr int NOALLOC_MIE_SLABS = 16;
 static __device__ __align__(256) double g_noalloc_tables[2 * (NOALLOC_GQ * (NOALLOC_GQ + 1) / 2) + 2 * 56];
+static __device__ __align__(256) double g_noalloc_mie[MIE_TAB];
 
 namespace {
 struct NoallocDevice {
   int ready = 0;
   char* scratch = nullptr;  // device address of g_noalloc_scratch
   double* tables = nullptr; // device address of g_noalloc_tables
+  double* mie_tab = nullptr; // device address of g_noalloc_mie
 };
 NoallocDevice g_noalloc_dev[64];
 std::mutex g_noalloc_mu;
@@ -1409,7 +1418,10 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
       void* sp = nullptr;
       void* tp = nullptr;
       if (cudaGetSymbolAddress(&sp, g_noalloc_scratch) != cudaSuccess) return PAMTRA_B200_FATAL;
-      if (cudaGetSymbolAddress(&tp, g_noalloc_tables) != cudaSuccess) return PAMTRA_B200_FATAL;
+      void* mp = nullptr;
+      if (cudaGetSymbolAddress(&tp, g_noalloc_tables) != cudaSuccess ||
+          cudaGetSymbolAddress(&mp, g_noalloc_mie) != cudaSuccess)
+        return PAMTRA_B200_FATAL;
       if (set_smem_attrs()) return PAMTRA_B200_FATAL;
       double* tab = (double*)tp;
       const size_t gqn = (size_t)NOALLOC_GQ * (NOALLOC_GQ + 1) / 2;
@@ -1436,7 +1448,9 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
           cudaMemcpyToSymbol(c_h2o_ws, H_H2O_WS, sizeof(H_H2O_WS)) ||
           cudaMemcpyToSymbol(c_h2o_xs, H_H2O_XS, sizeof(H_H2O_XS)))
         return PAMTRA_B200_FATAL;
+      k_mie_tables<<<NT_MAX - 1, 128, 0, stream>>>((double*)mp, tab);
       if (cudaStreamSynchronize(stream) != cudaSuccess) return PAMTRA_B200_FATAL;
+      D.mie_tab = (double*)mp;
       D.scratch = (char*)sp;
       D.tables = tab;
       D.ready = 1;
@@ -1488,7 +1502,7 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   w.seg_cnt = (int*)(A + pl.o_segcnt);
   w.spin_limit = tc::MBAR_SPIN_LIMIT;
   w.mie_slab = (double*)(A + pl.o_mieslab); w.mie_nslab = pl.mie_nslab;
-  w.gq_x = D.tables; w.gq_w = D.tables + gqn; w.gq_max = NOALLOC_GQ;
+  w.gq_x = D.tables; w.gq_w = D.tables + gqn; w.gq_max = NOALLOC_GQ; w.mie_tab = D.mie_tab;
   w.lob_mu = D.tables + 2 * gqn; w.lob_w = D.tables + 2 * gqn + 56;
   const size_t Lm = cc.max_nlyrs, Fm = cc.max_nfreq;
   // the scratch keeps the previous call's contents: clear what must start at zero
@@ -1508,7 +1522,7 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   if (nh > 0) {
     const size_t sm_mie = MIE_WARPS * sizeof(MieSmem);
     k_refr<<<(unsigned)(((size_t)std::max(1, pl.pmax) * Fm + 127) / 128), 128, 0, stream>>>(b, w, *st);
-    k_mie<MIE_GROUP><<<NOALLOC_MIE_SLABS / MIE_WARPS, 32 * MIE_WARPS, sm_mie, stream>>>(b, w, *st);
+    k_mie<1><<<NOALLOC_MIE_SLABS / MIE_WARPS, 32 * MIE_WARPS, sm_mie, stream>>>(b, w, *st);
   }
   if (mask & 1) {
     if (nh > 0) k_layer<8><<<sms, LayerCfg<8>::T, sizeof(LayerSmem<8>), stream>>>(b, w, *st, out->scatter_matrix);

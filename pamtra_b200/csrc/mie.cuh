@@ -17,12 +17,13 @@ constexpr int NQ_MAX = 256;   // Gauss points per series (nquad)
 constexpr int NT_MAX = 128;   // Mie terms per bin
 
 // Shared memory of one warp of k_mie: the phase-function sums of the
-// current species per quadrature point (P11, P12, P33) and the weights and
-// term counts of the bins of the current pass.
+// current species per quadrature point (P11, P12, P33), the weights of the
+// bins of the current pass and the terms of its groups of eight bins (a
+// multiple of 4).
 struct MieSmem {
   double sump[3][NQ_MAX];
-  double bw[32], bd[32];
-  int bn[32];
+  double bw[32];
+  int gn[4];
 };
 // Coefficient slab of one warp in global scratch: up to 32 bins x kmax rows
 // of (a_n, b_n); 4096 doubles hold 32 bins up to 32 terms (size parameters
@@ -39,6 +40,58 @@ constexpr int MIE_SLAB_WARPS_PER_SM = 16;  // slabs reserved per SM (caps the k_
 // divides; the products differ from the quotients in the last bit only).
 // c_mie_inv covers the Legendre orders too (l <= MAXNLEG - 1 > NT_MAX).
 __constant__ double c_mie_c[NT_MAX + 1], c_mie_inv[MAXNLEG];
+
+// Angular tables of a species whose largest bin has nt terms (nt < NT_MAX):
+// its quadrature has mie_nquad(nt) points, symmetric about 0, so only the
+// first mie_hq(nt) are tabulated.
+//   c_n (pi_n + tau_n), c_n (pi_n - tau_n) of mieangle, double2 [n / 4][angle, to
+//   a multiple of 8][n % 4] (n from 0 for the first term; zero past the last
+//   angle): a fragment of the phase-function sums is 512 contiguous bytes;
+//   P_l, double [angle][l], l = 0 .. mie_nlegen(nt).
+// The offsets of nt in doubles are c_mie_toff (P_l: [1]); both tables of all
+// nt are MIE_TAB doubles.
+__host__ __device__ constexpr int mie_nlegen(int nt) { return 2 * nt < MAXNLEG - 1 ? 2 * nt : MAXNLEG - 1; }
+__host__ __device__ constexpr int mie_nquad(int nt) { return (mie_nlegen(nt) + 2 * nt + 2) / 2; }
+__host__ __device__ constexpr int mie_hq(int nt) { return (mie_nquad(nt) + 1) / 2; }
+__host__ __device__ constexpr int mie_ptab(int nt) { return (nt + 3) / 4 * 4 * ((mie_hq(nt) + 7) / 8 * 8) * 2; }
+__host__ __device__ constexpr int mie_ltab(int nt) { return mie_hq(nt) * (mie_nlegen(nt) + 1); }
+constexpr size_t mie_tab_doubles() {
+  size_t n = 0;
+  for (int nt = 1; nt < NT_MAX; nt++) n += mie_ptab(nt) + mie_ltab(nt);
+  return n;
+}
+constexpr size_t MIE_TAB = mie_tab_doubles();
+static_assert(MIE_TAB < ((size_t)1 << 31), "int offsets");
+__constant__ int c_mie_toff[2][NT_MAX];
+
+// One block per nt = blockIdx.x + 1, one thread per angle; gx: the packed nodes.
+__global__ void __launch_bounds__(128) k_mie_tables(double* tab, const double* gx) {
+  const int nt = blockIdx.x + 1, hq = mie_hq(nt), hq8 = (hq + 7) / 8 * 8, nquad = mie_nquad(nt), nl = mie_nlegen(nt);
+  double2* const pt = reinterpret_cast<double2*>(tab + c_mie_toff[0][nt]);
+  double* const lt = tab + c_mie_toff[1][nt];
+  for (int i = threadIdx.x; i < hq8; i += blockDim.x) {
+    const double mu = i < hq ? gx[(size_t)nquad * (nquad - 1) / 2 + i] : 0.0;
+    double pin = 1.0, pim = 0.0;
+    for (int n = 1; n <= (nt + 3) / 4 * 4; n++) {
+      // tau_n = n mu pi_n - (n+1) pi_{n-1}, pi_{n+1} = ((2n+1) mu pi_n - (n+1) pi_{n-1}) / n
+      const double mp = mu * pin, q = (double)(n + 1) * pim;
+      const double taun = fma((double)n, mp, -q);
+      const double c = i < hq ? c_mie_c[n] : 0.0;
+      pt[((size_t)((n - 1) >> 2) * hq8 + i) * 4 + ((n - 1) & 3)] = make_double2(c * (pin + taun), c * (pin - taun));
+      const double tmp = pin;
+      pin = fma((double)(2 * n + 1), mp, -q) * c_mie_inv[n];
+      pim = tmp;
+    }
+    if (i >= hq) continue;
+    double p1 = 1.0, p2 = 0.0;
+    for (int l = 0; l <= nl; l++) {
+      const double p = l == 0 ? 1.0 : ((2 * l - 1) * mu * p1 - (l - 1) * p2) * c_mie_inv[l];
+      lt[(size_t)i * (nl + 1) + l] = p;
+      p2 = p1;
+      p1 = p;
+    }
+  }
+}
 
 // src/eps_water.f90:653-757 eps_water_tkc (T in degC, f in GHz)
 __device__ cplx eps_water_tkc(double T, double f) {
@@ -217,15 +270,17 @@ __device__ cplx eps_mix_m(cplx eps1, double mix_de) {
   return cmplx4(em_real, em_imag);  // CMPLX without KIND (eps_mix.f90:44)
 }
 
-// a / b as a conj(b) / |b|^2 (one division); the Mie coefficient
-// denominators stay within a few hundred orders of magnitude of 1, so |b|^2
-// neither overflows nor underflows.
-__device__ __forceinline__ cplx cdiv_rcp(cplx a, cplx b) {
-  const double s = 1.0 / (b.re * b.re + b.im * b.im);
-  return cmk((a.re * b.re + a.im * b.im) * s, (a.im * b.re - a.re * b.im) * s);
+// INT(x + 4 x**0.3334 + 2) of mie_spheres.f90.  The power in single precision
+// is good to 1e-4 here (x**0.3334 below 6); only where that could change the whole number
+// (one value in a thousand) does the double-precision one decide.
+__device__ __forceinline__ int mie_nstop(double x) {
+  const float xf = (float)x;
+  if (xf > 1e-30f && xf < 200.0f) {
+    const float v = xf + 4.0f * exp2f(0.3334f * log2f(xf)) + 2.0f, fr = v - floorf(v);
+    if (fr > 1e-3f && fr < 1.0f - 1e-3f) return (int)v;
+  }
+  return (int)(x + 4.0 * pow(x, F(0.3334f)) + 2);
 }
-
-__device__ __forceinline__ int mie_nstop(double x) { return (int)(x + 4.0 * pow(x, F(0.3334f)) + 2); }
 
 // Refractive indices of liquid water (nmlSet['liq_mod']) and ice of every
 // (present layer, frequency) item, ahead of k_mie (src/scatProperties.f90:
@@ -265,13 +320,14 @@ __device__ __noinline__ void miecalc_slab(int nterms, double x, cplx mn, double*
   const cplx yinv = cdiv(cmk(1.0, 0.0), y), minv = cdiv(cmk(1.0, 0.0), m);
   // downward recurrence d(n-1) = n/y - 1/(d(n) + n/y), d(nn) = 0; keep d(1..nterms)
   cplx d = cmk(0.0, 0.0);
+  double rn = nn;
 #pragma unroll 1
-  for (int n = nn; n >= 2; n--) {
-    const cplx ny = cscale(yinv, (double)n);
+  for (int n = nn; n >= 2; n--, rn -= 1.0) {
+    const cplx ny = cscale(yinv, rn);
     // 1 / z as conj(z) / |z|^2: one division on the recurrence's critical path
     const cplx z = cadd(d, ny);
-    const double s = 1.0 / (z.re * z.re + z.im * z.im);
-    d = cmk(ny.re - z.re * s, ny.im + z.im * s);
+    const double s = 1.0 / fma(z.re, z.re, z.im * z.im);
+    d = cmk(fma(-z.re, s, ny.re), fma(z.im, s, ny.im));
     if (n - 1 <= nterms) *reinterpret_cast<double2*>(col + (size_t)(n - 2) * ldc) = make_double2(d.re, d.im);
   }
   double sx, cx;
@@ -280,30 +336,46 @@ __device__ __noinline__ void miecalc_slab(int nterms, double x, cplx mn, double*
   const double xinv = 1.0 / x;
   double sum1 = 0.0, sum2 = 0.0;
   cplx sum3 = cmk(0.0, 0.0);
+  cplx xin = cmplx4(psin, -chin);
+  double sg = -1.0;  // (-1)^n
+  rn = 1.0;
+  double* next = col;
+  double2 dv = *reinterpret_cast<const double2*>(col);
+  // rn = n; conversions share the FP64 units' issue slots
 #pragma unroll 1
-  for (int n = 1; n <= nterms; n++) {
+  for (int n = 1; n <= nterms; n++, rn += 1.0) {
+    const double r21 = 2.0 * rn - 1.0, r23 = 2.0 * rn + 1.0;
     double tmp = psin;
-    psin = (2 * n - 1) * xinv * psin - psim;
+    psin = r21 * xinv * psin - psim;
     psim = tmp;
     tmp = chin;
-    chin = (2 * n - 1) * xinv * chin - chim;
+    chin = r21 * xinv * chin - chim;
     chim = tmp;
-    const cplx xin = cmplx4(psin, -chin), xim = cmplx4(psim, -chim);
-    double* row = col + (size_t)(n - 1) * ldc;
-    const double2 dv = *reinterpret_cast<const double2*>(row);
+    const cplx xim = xin;
+    xin = cmplx4(psin, -chin);
     const cplx dn = cmk(dv.x, dv.y);
-    cplx ctmp = cmul(dn, minv);
-    ctmp.re = ctmp.re + n * xinv;
-    const cplx an = cdiv_rcp(cmk(ctmp.re * psin - psim, ctmp.im * psin), csub(cmul(ctmp, xin), xim));
-    ctmp = cmul(m, dn);
-    ctmp.re = ctmp.re + n * xinv;
-    const cplx bn = cdiv_rcp(cmk(ctmp.re * psin - psim, ctmp.im * psin), csub(cmul(ctmp, xin), xim));
+    double* row = next;
+    next += ldc;
+    if (n < nterms) dv = *reinterpret_cast<const double2*>(next);  // travels during this term
+    // a_n and b_n: numerators over denominators z as (numerator conj(z)) / |z|^2, both by one
+    // reciprocal (|z| stays within a few hundred orders of magnitude of 1)
+    const double nx = rn * xinv;
+    const cplx ca = cmk(fma(dn.re, minv.re, fma(-dn.im, minv.im, nx)), fma(dn.re, minv.im, dn.im * minv.re));
+    const cplx cb = cmk(fma(m.re, dn.re, fma(-m.im, dn.im, nx)), fma(m.re, dn.im, m.im * dn.re));
+    const cplx pa = cmk(fma(ca.re, psin, -psim), ca.im * psin), pb = cmk(fma(cb.re, psin, -psim), cb.im * psin);
+    const cplx za = cmk(fma(ca.re, xin.re, fma(-ca.im, xin.im, -xim.re)), fma(ca.re, xin.im, fma(ca.im, xin.re, -xim.im)));
+    const cplx zb = cmk(fma(cb.re, xin.re, fma(-cb.im, xin.im, -xim.re)), fma(cb.re, xin.im, fma(cb.im, xin.re, -xim.im)));
+    const double qa = fma(za.re, za.re, za.im * za.im), qb2 = fma(zb.re, zb.re, zb.im * zb.im);
+    const double rq = 1.0 / (qa * qb2), ra = rq * qb2, rb = rq * qa;
+    const cplx an = cmk(fma(pa.re, za.re, pa.im * za.im) * ra, fma(pa.im, za.re, -(pa.re * za.im)) * ra);
+    const cplx bn = cmk(fma(pb.re, zb.re, pb.im * zb.im) * rb, fma(pb.im, zb.re, -(pb.re * zb.im)) * rb);
     *reinterpret_cast<double2*>(row) = make_double2(an.re + bn.re, an.im + bn.im);
     *reinterpret_cast<double2*>(row + 2) = make_double2(an.re - bn.re, an.im - bn.im);
-    sum1 = sum1 + (2 * n + 1) * (an.re + bn.re);
-    sum2 = sum2 + (2 * n + 1) * ((an.re * an.re - an.im * (-an.im)) + (bn.re * bn.re - bn.im * (-bn.im)));
-    const double fac = (double)((float)(2 * n + 1) * ((n & 1) ? -1.0f : 1.0f));
-    sum3 = cadd(sum3, cscale(csub(an, bn), fac));
+    sum1 = fma(r23, an.re + bn.re, sum1);
+    sum2 = fma(r23, fma(an.re, an.re, an.im * an.im) + fma(bn.re, bn.re, bn.im * bn.im), sum2);
+    const double r3 = r23 * sg;
+    sum3 = cmk(fma(an.re - bn.re, r3, sum3.re), fma(an.im - bn.im, r3, sum3.im));
+    sg = -sg;
   }
   qext = 2.0 / (x * x) * sum1;
   qscat = 2.0 / (x * x) * sum2;
@@ -311,103 +383,123 @@ __device__ __noinline__ void miecalc_slab(int nterms, double x, cplx mn, double*
   qback = t.re * sum3.re - t.im * (-sum3.im);
 }
 
-// Phase-matrix elements P11, P12 (= P21) and P33 of one angle, summed over
-// the bins j0 .. j0+GB-1 of a pass with their weights (mieangle,
-// mie_scat_utilities.f90:119-160, and the PSD sums of mie_spheres.f90:
-// 239-249).  With S+ = S1 + S2 = sum c_n u_n (pi_n + tau_n) and
-// S- = S1 - S2 = sum c_n v_n (pi_n - tau_n) each term costs two complex
-// multiply-adds instead of four, and
+// Phase B of one pass (whole warp): the phase-matrix elements P11, P12 (=
+// P21) and P33 of every angle, summed over the pass's bins with their weights
+// (mieangle, mie_scat_utilities.f90:119-160, and the PSD sums of
+// mie_spheres.f90:239-249).  With S+ = S1 + S2 = sum c_n u_n (pi_n + tau_n) and
+// S- = S1 - S2 = sum c_n v_n (pi_n - tau_n),
 //   P11 = (|S1|^2 + |S2|^2) / 2 = (|S+|^2 + |S-|^2) / 4,
 //   P12 = (|S2|^2 - |S1|^2) / 2 = -Re(S+ conj(S-)) / 2,
 //   P33 = Re(S2 conj(S1))       = (|S+|^2 - |S-|^2) / 4.
-// The pi_n / tau_n recurrence of the angle runs once for the group (rows
-// of bins without particles, and rows past a bin's own term count, hold
-// zeros).
-constexpr int MIE_GROUP = 4;  // default bins per work item (the launch shape chooses 4 or 8)
-template <int GB>
-__device__ __forceinline__ void mie_angle_group(const double* __restrict__ slab, int ldc, int j0, int nmax, double mu,
-                                                const double* __restrict__ wt, const double* __restrict__ dd, int nj,
-                                                double* sum0, double* sum1, double* sum2) {
-  double s[GB][4];  // S+ (re, im), S- (re, im)
-#pragma unroll
-  for (int j = 0; j < GB; j++) s[j][0] = s[j][1] = s[j][2] = s[j][3] = 0.0;
-  double pin = 1.0, pim = 0.0;
-  const double* row = slab + 4 * j0;
-  for (int n = 1; n <= nmax; n++, row += ldc) {
-    const double c = c_mie_c[n], rn = c_mie_inv[n];
-    // tau_n = n mu pi_n - (n+1) pi_{n-1}, pi_{n+1} = ((2n+1) mu pi_n - (n+1) pi_{n-1}) / n
-    const double mp = mu * pin, q = (double)(n + 1) * pim;
-    const double taun = fma((double)n, mp, -q);
-    const double cpl = c * (pin + taun), cmi = c * (pin - taun);
-#pragma unroll
-    for (int j = 0; j < GB; j++) {
-      const double2 u = *reinterpret_cast<const double2*>(row + 4 * j);
-      const double2 v = *reinterpret_cast<const double2*>(row + 4 * j + 2);
-      s[j][0] = fma(u.x, cpl, s[j][0]);
-      s[j][1] = fma(u.y, cpl, s[j][1]);
-      s[j][2] = fma(v.x, cmi, s[j][2]);
-      s[j][3] = fma(v.y, cmi, s[j][3]);
-    }
-    const double tmp = pin;
-    pin = fma((double)(2 * n + 1), mp, -q) * rn;
-    pim = tmp;
-  }
-  // add each bin's weighted elements to the angle's sums in bin order, so
-  // that the sums do not depend on the number of bins per work item
-  double a0 = sum0[0], a1 = sum1[0], a2 = sum2[0];
-#pragma unroll
-  for (int j = 0; j < GB; j++) {
-    if (j >= nj || !(wt[j] > 0.0)) continue;
-    const double ap = s[j][0] * s[j][0] + s[j][1] * s[j][1], am = s[j][2] * s[j][2] + s[j][3] * s[j][3];
-    const double p0 = 0.25 * (ap + am), p2 = 0.25 * (ap - am);
-    const double p1 = -0.5 * (s[j][0] * s[j][2] + s[j][1] * s[j][3]);
-    a0 = a0 + (p0 * wt[j]) * dd[j];
-    a1 = a1 + (p1 * wt[j]) * dd[j];
-    a2 = a2 + (p2 * wt[j]) * dd[j];
-  }
-  sum0[0] = a0;
-  sum1[0] = a1;
-  sum2[0] = a2;
-}
-
-// Phase B of one pass (whole warp): item u = g * nquad + i is angle i over
-// the bins of group g of the pass.  A round takes min(32, nquad) consecutive
-// items, so its angles are distinct and each lane adds into its angle's sums
-// without conflicts; rounds go in order, so every angle receives its bins in
-// bin order whatever the group size.  Out of line so that the kernel's state
-// is saved once per pass and the items keep the registers for their sums.
-template <int GB>
+// S+ and S- of eight bins at eight angles are four real products over the
+// terms: DMMAs, the bins' coefficients as the left fragments and the angular
+// table as the right ones.  pi_n + tau_n at -mu is (-1)^(n+1) times pi_n - tau_n
+// at mu, so a table fragment serves an angle tile and its mirror image: eight
+// DMMAs for four 16-byte loads.  A lane ends with S+ and S- of bin lane / 4
+// at two angles of each tile and weighs them without an exchange; the sum
+// over the eight bins of a group is one shuffle tree per tile and pass, so
+// the result does not depend on the launch shape.  Rows past a bin's terms and
+// bins without particles hold zeros.  NP tile pairs go together (a
+// coefficient fragment is read once for them).
+template <int NP>
 __device__ __noinline__ void mie_pass_sums(MieSmem& S, const double* __restrict__ slab, int ldc, int cb, int nquad,
-                                           const double* __restrict__ gx) {
-  const int lane = threadIdx.x & 31;
-  const int G = (cb + GB - 1) / GB;
-  const int nu = G * nquad;
-  const int W = min(32, nquad);
-  for (int u0 = 0; u0 < nu; u0 += W) {
-    const int u = u0 + lane;
-    if (lane < W && u < nu) {
-      const int g = u / nquad, i = u - g * nquad;
-      const int j0 = GB * g, nj = min(GB, cb - j0);
-      int nmax = 0;
-      for (int j = 0; j < nj; j++) nmax = max(nmax, S.bn[j0 + j]);
-      mie_angle_group<GB>(slab, ldc, j0, nmax, gx[i], S.bw + j0, S.bd + j0, nj, &S.sump[0][i], &S.sump[1][i],
-                          &S.sump[2][i]);
+                                           const double2* __restrict__ tab) {
+  const int lane = threadIdx.x & 31, g = lane >> 2, q = lane & 3;
+  const int hq = (nquad + 1) / 2, nt = (hq + 7) >> 3;
+  const int flip = (q & 1) << 31;  // sign of (-1)^(n+1) for the lane's terms n = 1 + 4 k + q
+  for (int t0 = 0; t0 < nt; t0 += NP) {
+    double ps[NP][2][2][3];
+#pragma unroll
+    for (int k = 0; k < NP * 12; k++) (&ps[0][0][0][0])[k] = 0.0;
+    for (int j0 = 0; j0 < cb; j0 += 8) {
+      const int nmax = S.gn[j0 >> 3];
+      if (nmax == 0) continue;
+      double acc[NP][2][4][2];
+#pragma unroll
+      for (int k = 0; k < NP * 16; k++) (&acc[0][0][0][0])[k] = 0.0;
+      const double* a = slab + 4 * (j0 + g) + q * ldc;
+      const double2* bt = tab + t0 * 32 + lane;
+      double2 u = *reinterpret_cast<const double2*>(a), v = *reinterpret_cast<const double2*>(a + 2);
+      double2 f[NP];
+#pragma unroll
+      for (int k = 0; k < NP; k++) f[k] = t0 + k < nt ? bt[k * 32] : make_double2(0.0, 0.0);
+      for (int n0 = 0; n0 < nmax; n0 += 4) {
+        const double2 uc = u, vc = v;
+        double2 fc[NP];
+#pragma unroll
+        for (int k = 0; k < NP; k++) fc[k] = f[k];
+        if (n0 + 4 < nmax) {  // the next four terms travel while these multiply
+          a += 4 * ldc;
+          bt += nt * 32;
+          u = *reinterpret_cast<const double2*>(a);
+          v = *reinterpret_cast<const double2*>(a + 2);
+#pragma unroll
+          for (int k = 0; k < NP; k++)
+            if (t0 + k < nt) f[k] = bt[k * 32];
+        }
+#pragma unroll
+        for (int k = 0; k < NP; k++) {
+          const double mx = __hiloint2double(__double2hiint(fc[k].y) ^ flip, __double2loint(fc[k].y));
+          const double my = __hiloint2double(__double2hiint(fc[k].x) ^ flip, __double2loint(fc[k].x));
+          dmma(acc[k][0][0], uc.x, fc[k].x);
+          dmma(acc[k][0][1], uc.y, fc[k].x);
+          dmma(acc[k][0][2], vc.x, fc[k].y);
+          dmma(acc[k][0][3], vc.y, fc[k].y);
+          dmma(acc[k][1][0], uc.x, mx);
+          dmma(acc[k][1][1], uc.y, mx);
+          dmma(acc[k][1][2], vc.x, my);
+          dmma(acc[k][1][3], vc.y, my);
+        }
+      }
+      const double wd = S.bw[j0 + g];
+#pragma unroll
+      for (int k = 0; k < NP; k++)
+#pragma unroll
+        for (int m = 0; m < 2; m++)
+#pragma unroll
+          for (int e = 0; e < 2; e++) {
+            const double s0 = acc[k][m][0][e], s1 = acc[k][m][1][e], s2 = acc[k][m][2][e], s3 = acc[k][m][3][e];
+            const double ap = s0 * s0 + s1 * s1, am = s2 * s2 + s3 * s3;
+            ps[k][m][e][0] = fma(0.25 * (ap + am), wd, ps[k][m][e][0]);
+            ps[k][m][e][1] = fma(-0.5 * (s0 * s2 + s1 * s3), wd, ps[k][m][e][1]);
+            ps[k][m][e][2] = fma(0.25 * (ap - am), wd, ps[k][m][e][2]);
+          }
     }
-    __syncwarp();
+#pragma unroll
+    for (int k = 0; k < NP; k++)
+#pragma unroll
+      for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int i = (t0 + k) * 8 + 2 * q + e, im = m ? nquad - 1 - i : i;
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            double x = ps[k][m][e][c];
+#pragma unroll
+            for (int o = 4; o < 32; o <<= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+            if (g == c && i < hq && (m == 0 || im != i)) S.sump[c][im] += x;
+          }
+        }
   }
+  __syncwarp();
 }
 
 // One warp per (present layer, frequency) item; species loop in descriptor
 // order.  src/scatProperties.f90:62-1002 (mie-sphere branch and the species
 // sums :920-949, finalize :993) with src/mie_spheres.f90:14-345 per species.
 // Per species the bins go in passes of up to 32: lanes over bins compute
-// the Mie coefficients into the warp's slab (phase A), then lanes over
-// (group of bins, angle) work items form the phase-function sums of
-// the pass (phase B); each round of 32 items adds into the per-angle sums
-// in lane order, so every result is independent of the launch shape.  The
-// Legendre projection runs lanes over quadrature points with shuffle sums.
+// the Mie coefficients into the warp's slab (phase A), then the
+// phase-function sums of the pass are formed on the FP64 tensor cores (phase B,
+// mie_pass_sums).  The Legendre projection runs lanes over orders, the
+// quadrature points folded about 0 (P_l is even or odd) and P_l from a table.
 // The species sums accumulate in the item's coefficient output row.
-template <int GB>
+// Bound by the FP64 pipes, which the scalar series of phase A and the DMMAs of
+// phase B share, and by the latency of both at 16 warps per SM (128 registers):
+// Mie stage at 1500 columns of 6-term species 6.8 ms with FP64 FMAs per (four
+// bins, angle) and warp sums per Legendre order, now 4.9 ms; 40 columns of
+// 20-term species with 200 bins 6.2 ms, now 3.6 ms.
+// One tile pair (NP = 1); two spill (8.2 and 6.0 ms before the series were trimmed).
+template <int NP>
 __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_settings st) {
   extern __shared__ double smem_raw[];
   MieSmem& S = reinterpret_cast<MieSmem*>(smem_raw)[threadIdx.x >> 5];
@@ -459,8 +551,6 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
       // density / diameter of bin i (frequency-dependent soft spheroids of
       // make_soft_spheroid.f90:109-114 resolved here)
       auto dens_diam = [&](int i, double& rho, double& dia) {
-        rho = brho[i];
-        dia = bd[i];
         if (rho == -1.0) {
           const double mind = st.hydro_softsphere_min_density;
           rho = (sp_as_ratio == -20.) ? 0.863 * freq + 115.0 : 0.815 * freq + 11.2;
@@ -472,7 +562,7 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
           }
         }
       };
-      double rhoN, diaN;
+      double rhoN = brho[nb - 1], diaN = bd[nb - 1];
       dens_diam(nb - 1, rhoN, diaN);
       const double xmax = PI * diaN / wl;
       const int nterms = mie_nstop(xmax);
@@ -482,22 +572,26 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
         status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;
         break;
       }
-      const double* gx = w.gq_x + (size_t)nquad * (nquad - 1) / 2;
       const double* gw = w.gq_w + (size_t)nquad * (nquad - 1) / 2;
+      const double2* ptab = reinterpret_cast<const double2*>(w.mie_tab + c_mie_toff[0][nterms]);
+      const double* ltab = w.mie_tab + c_mie_toff[1][nterms];
       for (int i = lane; i < nquad; i += 32) { S.sump[0][i] = 0; S.sump[1][i] = 0; S.sump[2][i] = 0; }
-      // rows the slab needs: every active bin's own series length, at least nterms
-      int kmax = nterms;
+      // rows the slab needs: the series of the largest bin (one more than its
+      // length, which rounding could have below that of a smaller bin)
+      double dmax = diaN;
+#pragma unroll 2
       for (int ir = lane; ir < nb; ir += 32) {
-        if (bnd[ir] / bdd[ir] > 0) {
-          double rho, dia;
-          dens_diam(ir, rho, dia);
-          kmax = max(kmax, min(mie_nstop(PI * dia / wl), NT_MAX - 1));
-        }
+        const double nd = bnd[ir];
+        double rho = brho[ir], dia = bd[ir];
+        dens_diam(ir, rho, dia);
+        dmax = fmax(dmax, nd != 0.0 ? dia : 0.0);
       }
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1) kmax = max(kmax, __shfl_xor_sync(0xffffffffu, kmax, o));
-      // bins per pass, a multiple of the group size so that no group runs past the slab's columns
-      const int bp = min(32, MIE_SLAB / (4 * kmax)) & ~(GB - 1);
+      for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
+      int kmax = max(nterms, dmax > diaN ? min(mie_nstop(PI * dmax / wl) + 1, NT_MAX - 1) : min(nterms + 1, NT_MAX - 1));
+      kmax = (kmax + 3) & ~3;  // terms go in fours
+      // bins per pass, a multiple of a group's eight so that no group runs past the slab's columns
+      const int bp = min(32, MIE_SLAB / (4 * kmax)) & ~7;
       const int ldc = 4 * bp;
       __syncwarp();
       double sqe = 0.0, sqs = 0.0, sqb = 0.0;
@@ -511,9 +605,9 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
           double* col = slab + 4 * lane;
           if (lane < cb) {
             deld = bdd[ir];
+            double rho = brho[ir], dia = bd[ir];
             ndens = bnd[ir] / deld;
             if (ndens > 0) {
-              double rho, dia;
               dens_diam(ir, rho, dia);
               const cplx ms = (sp_liq_ice == -1 && rho != 917.0) ? eps_mix_m(m_ice, rho) : m_ice;
               const double x = PI * dia / wl;
@@ -539,15 +633,22 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
             // src/scatProperties.f90:916 (0 / 0 = NaN for an empty bin)
             if (bscat && ir < w.psd_nbin) bscat[s_idx * (size_t)w.psd_nbin + ir] = qb_bin / ndens;
           }
-          for (int n = nm; n < nterms; n++)
-            *reinterpret_cast<double4*>(col + (size_t)n * ldc) = make_double4(0.0, 0.0, 0.0, 0.0);
-          S.bw[lane] = wgt;
-          S.bd[lane] = deld;
-          S.bn[lane] = nm;
+          // terms of the group (bp lanes, a multiple of eight, are here)
+          const unsigned bins = bp == 32 ? 0xffffffffu : (1u << bp) - 1;
+          int gn = nm;
+#pragma unroll
+          for (int o = 1; o < 8; o <<= 1) gn = max(gn, __shfl_xor_sync(bins, gn, o));
+          gn = (gn + 3) & ~3;
+          for (int n = nm; n < gn; n++) {
+            *reinterpret_cast<double2*>(col + (size_t)n * ldc) = make_double2(0.0, 0.0);
+            *reinterpret_cast<double2*>(col + (size_t)n * ldc + 2) = make_double2(0.0, 0.0);
+          }
+          S.bw[lane] = wgt * deld;
+          if ((lane & 7) == 0) S.gn[lane >> 3] = gn;
         }
         __syncwarp();
         // ---- phase B: the phase-function sums of the pass
-        mie_pass_sums<GB>(S, slab, ldc, cb, nquad, gx);
+        mie_pass_sums<NP>(S, slab, ldc, cb, nquad, ptab);
       }
       sqe = warp_sum(sqe);
       sqs = warp_sum(sqs);
@@ -556,59 +657,51 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
       const double scatter = sqs;
       const double salb_h = scatter / extinction;
       const double tmp = (wl * wl / (PI * scatter));
-      for (int i = lane; i < nquad; i += 32) {
-        const double wt = gw[i];
+      // weigh the points and fold them about 0: i < nquad / 2 holds s(i) +
+      // s(mirror), the mirrored places s(i) - s(mirror)
+      const int hq = (nquad + 1) / 2;
+      for (int i = lane; i < hq; i += 32) {
+        const int im = nquad - 1 - i;
+        const double wt = gw[i], wm = gw[im];
 #pragma unroll
-        for (int k = 0; k < 3; k++) S.sump[k][i] = tmp * S.sump[k][i] * wt;
+        for (int k = 0; k < 3; k++) {
+          const double x = tmp * S.sump[k][i] * wt, y = im != i ? tmp * S.sump[k][im] * wm : 0.0;
+          S.sump[k][i] = x + y;
+          if (im != i) S.sump[k][im] = x - y;
+        }
       }
       __syncwarp();
       // Legendre projection: coef_l = sum_i sump(i) P_l(mu_i), l = 0..nlegen,
-      // in chunks of 64 quadrature points (two per lane); the chunk sums of
-      // each order go into the slab (legh), in chunk order
+      // lane over orders (64 at a time), into the slab (legh)
       double* const legh = slab;  // [3][MAXNLEG]; the coefficients of the pass are no longer needed
       const double thr = F(1.0e-7f);
-      for (int q0 = 0; q0 < nquad; q0 += 64) {
-        const int i0 = q0 + lane, i1 = q0 + 32 + lane;
-        const double mu0 = (i0 < nquad) ? gx[i0] : 0.0, mu1 = (i1 < nquad) ? gx[i1] : 0.0;
-        double s0[3], s1[3];
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          s0[k] = (i0 < nquad) ? S.sump[k][i0] : 0.0;
-          s1[k] = (i1 < nquad) ? S.sump[k][i1] : 0.0;
-        }
-        double pa = 1.0, pa1 = 1.0, pa2 = 0.0, pb = 1.0, pb1 = 1.0, pb2 = 0.0;
-        for (int l = 0; l <= nlegen; l++) {
-          if (l > 0) {
-            pa = ((2 * l - 1) * mu0 * pa1 - (l - 1) * pa2) * c_mie_inv[l];
-            pb = ((2 * l - 1) * mu1 * pb1 - (l - 1) * pb2) * c_mie_inv[l];
-          }
-          double acc[3];
-#pragma unroll
-          for (int k = 0; k < 3; k++) acc[k] = fma(s1[k], pb, fma(s0[k], pa, 0.0));
-          pa2 = pa1;
-          pa1 = pa;
-          pb2 = pb1;
-          pb1 = pb;
-#pragma unroll
-          for (int k = 0; k < 3; k++) acc[k] = warp_sum(acc[k]);
-          if (lane == 0) {
-#pragma unroll
-            for (int k = 0; k < 3; k++) legh[k * MAXNLEG + l] = (q0 == 0) ? acc[k] : legh[k * MAXNLEG + l] + acc[k];
-          }
-        }
-      }
-      // orders past this species' series are zero in the species sums (mie_spheres.f90:309-316)
-      for (int l = nlegen + 1 + lane; l < MAXNLEG; l += 32) {
-#pragma unroll
-        for (int k = 0; k < 3; k++) legh[k * MAXNLEG + l] = 0.0;
-      }
-      __syncwarp();
       int last = -1;
-      for (int l = lane; l <= nlegen; l += 32) {
-        const double fac = (double)((float)(2 * l + 1) / 2.0f);  // REAL(4) division, exact
+      for (int l0 = 0; l0 <= nlegen; l0 += 64) {
+        const int l = l0 + lane;
+        double acc[2][3] = {{0.0, 0.0, 0.0}, {0.0, 0.0, 0.0}};
+        // odd orders read the differences (the middle point of an odd rule has none)
+        const int step = (l & 1) ? -1 : 1, n = (l & 1) ? nquad / 2 : hq;
+        const double *sp = &S.sump[0][0] + ((l & 1) ? nquad - 1 : 0), *tp = ltab + l;
+        const bool in0 = l <= nlegen, in1 = l + 32 <= nlegen;
+#pragma unroll 4
+        for (int i = 0; i < n; i++, sp += step, tp += nlegen + 1) {
+          const double p0 = in0 ? tp[0] : 0.0, p1 = in1 ? tp[32] : 0.0;
 #pragma unroll
-        for (int k = 0; k < 3; k++) legh[k * MAXNLEG + l] = fac * legh[k * MAXNLEG + l];
-        if (legh[l] > thr) last = l;
+          for (int k = 0; k < 3; k++) {
+            const double x = sp[k * NQ_MAX];
+            acc[0][k] = fma(x, p0, acc[0][k]);
+            acc[1][k] = fma(x, p1, acc[1][k]);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+          const int lj = l + 32 * j;
+          if (lj > nlegen) continue;
+          const double fac = (double)((float)(2 * lj + 1) / 2.0f);  // REAL(4) division, exact
+#pragma unroll
+          for (int k = 0; k < 3; k++) legh[k * MAXNLEG + lj] = fac * acc[j][k];
+          if (fac * acc[j][0] > thr) last = lj;
+        }
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) last = max(last, __shfl_xor_sync(0xffffffffu, last, o));
@@ -628,7 +721,8 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
       for (int jj = lane; jj < nlegen_coef; jj += 32) {
 #pragma unroll
         for (int k = 0; k < 3; k++)
-          legc[k * MAXNLEG + jj] = legc[k * MAXNLEG + jj] + (legh[k * MAXNLEG + jj] * salb_h * extinction);
+          // orders past this species' series are zero (mie_spheres.f90:309-316)
+          legc[k * MAXNLEG + jj] = legc[k * MAXNLEG + jj] + ((jj <= nlegen ? legh[k * MAXNLEG + jj] : 0.0) * salb_h * extinction);
       }
       __syncwarp();
       if (nlegen_coef > MAXNLEG - 1) { status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE; break; }

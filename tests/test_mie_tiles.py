@@ -1,0 +1,51 @@
+"""Mie sums where the tiles of k_mie have remainders: bins around groups of
+eight and passes of 32, series of about 5 to 60 terms (fours; 64 Legendre
+orders per chunk; odd and even numbers of angle tiles; passes of fewer than 32
+bins), against the oracle; and the two tile shapes against each other.
+Tolerance: that of all single-scattering outputs, 1e-9 relative.
+"""
+import numpy as np
+import pytest
+import test_single_scattering_parity as ssp
+
+from pamtra_b200 import batch as pbatch
+from pamtra_b200 import packing
+from pamtra_b200 import workloads as wl
+
+pytestmark = pytest.mark.gpu
+FREQS = [5.0, 31.4, 53.0, 89.0, 157.0, 190.31, 243.0, 325.0, 448.0]
+
+
+def _batch(nbins, nlay=5, seed=41):
+    rng = np.random.default_rng(seed)
+    kinds = ["rwc", "swc", "gwc", "iwc"]
+    sp = np.empty(4, dtype=packing.SPECIES_DTYPE)
+    for j, k in enumerate(kinds):
+        sp[j] = wl._species_row(k, np.random.default_rng(300 + j), nbin=nbins[j], gamma=(k != "rwc"), rho=400.0)
+    qs = [[10 ** rng.uniform(-4.0, -2.7) for _ in kinds]]
+    b = wl._packed(wl._settings(16), sp, 0, np.array([nlay]), [FREQS], None, [kinds], qs, np.array([9000.0]), rng, nlay,
+                   4, False)
+    b.host["temp_lev"][0, :nlay + 1] = np.linspace(295.0, 245.0, nlay + 1)
+    return b
+
+
+@pytest.mark.parametrize("nbins", [(2, 7, 8, 9), (31, 32, 33, 40), (24, 25, 64, 65)])
+def test_mie_tiles_match_oracle(oracle_mod, native, nbins):
+    import torch
+    dev = torch.device("cuda", 0)
+    b = _batch(nbins)
+    out = ssp._outputs(b, dev)
+    pbatch.run(b, 0, out)
+    torch.cuda.synchronize()
+    assert ssp._compare(b, out, oracle_mod, 16) >= 9
+    eng = native.engine(0)
+    keep = eng.get_launch()
+    try:
+        eng.set_launch((2, 0, 0, 0, 8))
+        two = ssp._outputs(b, dev)
+        pbatch.run(b, 0, two)
+        torch.cuda.synchronize()
+    finally:
+        eng.set_launch(keep)
+    for k in ("kexttot", "salbedo", "scatter_matrix", "tb"):
+        assert torch.equal(out[k], two[k]), k
