@@ -958,15 +958,15 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
     else k_mie<1><<<g, 32 * mw, sm_mie, stream>>>(b, w, *st);
     launches++;
     if (w.wtab[0] && (mask & 1)) {
-      k_scat_weights<8><<<SCAT_NPI * ((2 * 8 * 8 + 127) / 128), 128, 0, stream>>>(ctx->wtab[0], w.wt_need, w.wt_ready, ctx->lob_mu);
+      k_scat_weights<8><<<SCAT_NPI * ((scat_pairs(8) + 127) / 128), 128, 0, stream>>>(ctx->wtab[0], w.wt_need, w.wt_ready, ctx->lob_mu);
       launches++;
     }
     if (w.wtab[1] && (mask & 2)) {
-      k_scat_weights<16><<<SCAT_NPI * ((2 * 16 * 16 + 127) / 128), 128, 0, stream>>>(ctx->wtab[1], w.wt_need, w.wt_ready, ctx->lob_mu);
+      k_scat_weights<16><<<SCAT_NPI * ((scat_pairs(16) + 127) / 128), 128, 0, stream>>>(ctx->wtab[1], w.wt_need, w.wt_ready, ctx->lob_mu);
       launches++;
     }
     if (w.wtab[2] && (mask & 4)) {
-      k_scat_weights<32><<<SCAT_NPI * ((2 * 32 * 32 + 127) / 128), 128, 0, stream>>>(ctx->wtab[2], w.wt_need, w.wt_ready, ctx->lob_mu);
+      k_scat_weights<32><<<SCAT_NPI * ((scat_pairs(32) + 127) / 128), 128, 0, stream>>>(ctx->wtab[2], w.wt_need, w.wt_ready, ctx->lob_mu);
       launches++;
     }
   }

@@ -79,7 +79,7 @@ struct Work {
   float* add_stk;                      // [C*Fm][STK_FLOATS] FP32 adding stacks, k_adding_tc -> k_adding_finish
   int* seg_cnt;                        // [C*Fm] segments of the unit k_adding has finished (zero at the start)
   // scatcnv weight tables per NUMMU index (0: N = 8, 1: 16, 2: 32); null = direct sums
-  const double* wtab[3];               // [numpts index][l][5][2 N^2], see scat_weight_offset
+  const double* wtab[3];               // [numpts index][l][5][scat_pairs(N)], see scat_weight_offset
   int* wt_need;                        // [3][SCAT_NPI] numpts values seen (set by k_mie)
   int* wt_ready;                       // [3][SCAT_NPI] tables already computed
   // polls of each wait on a tensor-core MMA before it gives up (PAMTRA_B200_ST_TIMEOUT)
@@ -103,11 +103,12 @@ __host__ __device__ __forceinline__ int nmu_index(int N) { return N == 8 ? 0 : (
 
 // scatcnv weight tables: numpts = 2 * ((nlegen + 1) / 2) + 4 takes SCAT_NPI
 // values 4, 6, ..., 204 (index pi = (numpts - 4) / 2); the table of pi holds
-// numpts - 3 = 2 pi + 1 Legendre orders x 5 weights x 2 N^2 (mu1, mu2) pairs,
-// so it starts 10 N^2 pi^2 doubles into the tables of N.
+// numpts - 3 = 2 pi + 1 Legendre orders x 5 weights x scat_pairs(N) angle pairs
+// mu1 <= mu2, so it starts 5 scat_pairs(N) pi^2 doubles into the tables of N.
 constexpr int SCAT_NPI = 101;
+__host__ __device__ constexpr int scat_pairs(int N) { return N * (N + 1) / 2; }
 __host__ __device__ __forceinline__ size_t scat_weight_offset(int N, int pi) {
-  return (size_t)10 * N * N * pi * pi;
+  return (size_t)5 * scat_pairs(N) * pi * pi;
 }
 __host__ __device__ __forceinline__ size_t scat_weight_doubles(int N) { return scat_weight_offset(N, SCAT_NPI); }
 

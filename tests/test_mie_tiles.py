@@ -49,3 +49,31 @@ def test_mie_tiles_match_oracle(oracle_mod, native, nbins):
         eng.set_launch(keep)
     for k in ("kexttot", "salbedo", "scatter_matrix", "tb"):
         assert torch.equal(out[k], two[k]), k
+
+
+@pytest.mark.parametrize("nummu", [8, 32])
+def test_phase_matrices_of_even_and_odd_series(oracle_mod, native, nummu):
+    """scatcnv from the pair table: the frequencies give species series of even
+    and odd length; 36 and 528 angle pairs, one and three per thread.  A
+    frequency whose phase function the angles do not resolve fails CHECK_NORM4
+    on both sides."""
+    import copy
+
+    import torch
+    dev = torch.device("cuda", 0)
+    b = _batch((8, 8, 16, 8), nlay=3)
+    st = copy.copy(wl._settings(nummu))
+    passed = 0
+    for f in FREQS:
+        one = pbatch.pack_columns(st, b.species, dict(b.host, freqs=np.array([f]), max_nfreq=1),
+                                  b.species_stride)
+        out = ssp._outputs(one, dev)
+        pbatch.run(one, 0, out)
+        torch.cuda.synchronize()
+        err = oracle_mod.run_column(oracle_mod.settings(st), one.species, one.host, 0, [f])[0]
+        if err:
+            assert int(out["status"][0, 0]) == (2 | native.ST_NORM)
+            continue
+        assert ssp._compare(one, out, oracle_mod, nummu) >= 1
+        passed += 1
+    assert passed >= 5
