@@ -101,7 +101,7 @@ struct TcSetupSmem {
   double az[2 * KMAX];
   double lin[2 * n], cst[2 * n];
   double mu[16], wq[16], nrm[16];
-  int item, stat;
+  int item;
   __device__ __forceinline__ double* mat(int i) { return i == 0 ? r : i == 1 ? t : i == 4 ? az : coef; }
 };
 

@@ -43,7 +43,7 @@ struct Tc64Setup {
   double az[2 * KMAX];
   double lin[2 * n], cst[2 * n];
   double mu[32], wq[32], nrm[32];
-  int item, stat;
+  int item;
   __device__ __forceinline__ double* mat(int i) { return i == 0 ? r : i == 1 ? t : i == 4 ? az : coef; }
 };
 

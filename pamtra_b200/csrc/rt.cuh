@@ -68,7 +68,7 @@ struct LayerSmem {
   double sc[n], is[n];            // sqrt(mu w) per row and its inverse
   double fro[n / 8];              // sums of squares of the scaled R, per warp
   InvScratch<n> inv;
-  int item, stat;
+  int item;
   // set-up buffers (layer_setup): 0 R, 1 T, 2 coefficients, 4 azimuth table
   __device__ __forceinline__ double* mat(int k) {
     return m + (k < 2 ? k * LMAT : 2 * LMAT + (k == 4 ? COEF : 0));
@@ -173,11 +173,18 @@ struct LayerItem {
 // INITIAL_SOURCE4 of one (present layer, frequency) item: leaves the
 // thin-layer R (S.m[0]) and T (S.m[1]) and the sources S.lin / S.cst in
 // shared memory.  Returns false when the item is not for this N.
+// Latency of one CTA, while its neighbours double: the table rows of several
+// orders travel at once, the Planck functions run in the last warp beside the
+// coefficients, norms eight lanes to a row. 
+// Set-up of an item of 1500 columns (N = 16) 46 k -> 23 k cycles, of a Mie-heavy one
+// 62 k -> 29 k; layer stage 22.0 -> 21.8 ms, mixed NUMMU 19.7 -> 19.4 (split
+// form 14.2 -> 13.7), split form 13.0 -> 12.85: the doubling of the others takes up the rest.
 template <int N, class SM, int T = RTCfg<N>::T>
 __device__ __forceinline__ bool layer_setup(const Batch& b, const Work& w, const pamtra_b200_settings& st,
                                             double* __restrict__ ssp_scat, SM& S, int item,
                                             LayerItem& it) {
   constexpr int n = RTCfg<N>::n, LD = RTCfg<N>::LD, MAT = RTCfg<N>::MAT;
+  static_assert(T == 8 * N, "eight threads per angle");
   const int t = threadIdx.x;
   const int Lm = b.max_nlyrs, Fm = b.max_nfreq;
     const int p = item / Fm, fi = item % Fm;
@@ -190,7 +197,8 @@ __device__ __forceinline__ bool layer_setup(const Batch& b, const Work& w, const
     const double* tl = w.temp_lev + (size_t)c * (Lm + 1);
     const double zdiff = fabs(hl[z + 1] - hl[z]);
     const double gas = fmax(w.kgas[((size_t)c * Fm + fi) * Lm + z], 0.0);
-    const double planck0 = planck(tl[z + 1], wl), planck1 = planck(tl[z], wl);
+    // Planck functions at the layer's upper and lower boundary, for now in S.lin
+    if (t >= T - 2) S.lin[T - 1 - t] = planck(tl[z + (T - 1 - t)], wl);
     const int nleg = w.m_nleg[item];
     const double kext = w.m_kext[item], salb = w.m_salb[item];
     double* Rb = S.mat(0);
@@ -220,43 +228,20 @@ __device__ __forceinline__ bool layer_setup(const Batch& b, const Work& w, const
       if (W) {
         // phase matrices from the azimuth weight tables (k_scat_weights)
         team_sync();
-        constexpr int C2 = scat_pairs(N), CPT = (C2 + T - 1) / T;
-        const double* Wp = W + scat_weight_offset(N, (numpts - 4) / 2) + t;
-        double acc[CPT][2][5];  // sums of the five weights over even and odd l
-#pragma unroll
-        for (int u = 0; u < CPT; u++)
-#pragma unroll
-          for (int e = 0; e < 10; e++) (&acc[u][0][0])[e] = 0.0;
-        auto order = [&](int l, int par) {
-          const double c0 = coef[l], c1 = coef[MAXNLEG + l], c2 = coef[2 * MAXNLEG + l];
-          const double* Wl = Wp + (size_t)l * 5 * C2;
-#pragma unroll
-          for (int u = 0; u < CPT; u++) {
-            if (t + u * T >= C2) continue;
-            const double* Wc = Wl + u * T;
-            acc[u][par][0] = fma(c0, Wc[0], acc[u][par][0]);
-            acc[u][par][1] = fma(c1, Wc[C2], acc[u][par][1]);
-            acc[u][par][2] = fma(c1, Wc[2 * C2], acc[u][par][2]);
-            acc[u][par][3] = fma(c0, Wc[3 * C2], acc[u][par][3]);
-            acc[u][par][4] = fma(c2, Wc[4 * C2], acc[u][par][4]);
-          }
-        };
-        for (int l = 0; l <= nleg; l += 2) {
-          order(l, 0);
-          if (l < nleg) order(l + 1, 1);
-        }
-#pragma unroll
-        for (int u = 0; u < CPT; u++) {
-          const int pair = t + u * T;
-          if (pair >= C2) continue;
+        // thread per angle pair in rounds of T; a remainder of up to T / 16 pairs
+        // takes sixteen threads each, over the orders
+        constexpr int C2 = scat_pairs(N), REST = C2 % T;
+        constexpr bool SPREAD = REST > 0 && REST * 16 <= T;
+        constexpr int CPT = C2 / T + (REST > 0 && !SPREAD ? 1 : 0), LS = CPT > 1 ? 2 : 4;
+        const double* Wp = W + scat_weight_offset(N, (numpts - 4) / 2);
+        auto store = [&](int pair, const double (&ev)[5], const double (&od)[5]) {
           const int j2 = scat_pair_row(pair), j1 = pair - j2 * (j2 + 1) / 2;
 #pragma unroll
           for (int q = 0; q < 2; q++) {
             double* Qm = (q == 0) ? Tb : Rb;
             double p[5];
 #pragma unroll
-            for (int e = 0; e < 5; e++)
-              p[e] = q == 0 ? acc[u][0][e] + acc[u][1][e] : acc[u][0][e] - acc[u][1][e];
+            for (int e = 0; e < 5; e++) p[e] = q == 0 ? ev[e] + od[e] : ev[e] - od[e];
             const double p22 = q == 0 ? p[3] + p[4] : p[3] - p[4];
             const int a = 2 * j1, b2 = 2 * j2;
             Qm[a * LD + b2] = p[0];
@@ -270,6 +255,68 @@ __device__ __forceinline__ bool layer_setup(const Batch& b, const Work& w, const
               Qm[(b2 + 1) * LD + a + 1] = p22;
             }
           }
+        };
+        const int r = t & 15, rest = C2 - REST + min(t >> 4, REST - 1);
+        double x[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+        if (SPREAD && r <= nleg) {
+#pragma unroll
+          for (int e = 0; e < 5; e++) x[e] = Wp[((size_t)r * 5 + e) * C2 + rest];
+        }
+        double acc[CPT > 0 ? CPT : 1][2][5];  // sums of the five weights over even and odd l
+#pragma unroll
+        for (int u = 0; u < CPT; u++)
+#pragma unroll
+          for (int e = 0; e < 10; e++) (&acc[u][0][0])[e] = 0.0;
+        for (int l0 = 0; l0 <= nleg; l0 += LS) {
+          double v[LS][CPT][5];
+#pragma unroll
+          for (int k = 0; k < LS; k++) {
+            const double* Wl = Wp + (size_t)min(l0 + k, nleg) * 5 * C2;
+#pragma unroll
+            for (int u = 0; u < CPT; u++)
+#pragma unroll
+              for (int e = 0; e < 5; e++) v[k][u][e] = Wl[e * C2 + min(t + u * T, C2 - 1)];
+          }
+#pragma unroll
+          for (int k = 0; k < LS; k++) {
+            const int l = l0 + k;
+            if (l > nleg) break;
+            const double c0 = coef[l], c1 = coef[MAXNLEG + l], c2 = coef[2 * MAXNLEG + l];
+#pragma unroll
+            for (int u = 0; u < CPT; u++) {
+              double(&a)[5] = acc[u][k & 1];
+              a[0] = fma(c0, v[k][u][0], a[0]);
+              a[1] = fma(c1, v[k][u][1], a[1]);
+              a[2] = fma(c1, v[k][u][2], a[2]);
+              a[3] = fma(c0, v[k][u][3], a[3]);
+              a[4] = fma(c2, v[k][u][4], a[4]);
+            }
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < CPT; u++)
+          if (t + u * T < C2) store(t + u * T, acc[u][0], acc[u][1]);
+        if (SPREAD) {
+          double sum[5] = {0.0, 0.0, 0.0, 0.0, 0.0}, other[5];
+          for (int l = r; l <= nleg; l += 16) {
+            if (l > r) {
+#pragma unroll
+              for (int e = 0; e < 5; e++) x[e] = Wp[((size_t)l * 5 + e) * C2 + rest];
+            }
+            const double c0 = coef[l], c1 = coef[MAXNLEG + l], c2 = coef[2 * MAXNLEG + l];
+            sum[0] = fma(c0, x[0], sum[0]);
+            sum[1] = fma(c1, x[1], sum[1]);
+            sum[2] = fma(c1, x[2], sum[2]);
+            sum[3] = fma(c0, x[3], sum[3]);
+            sum[4] = fma(c2, x[4], sum[4]);
+          }
+#pragma unroll
+          for (int e = 0; e < 5; e++) {
+#pragma unroll
+            for (int o = 2; o < 16; o <<= 1) sum[e] += __shfl_xor_sync(0xffffffffu, sum[e], o);
+            other[e] = __shfl_xor_sync(0xffffffffu, sum[e], 1);
+          }
+          if (r == 0 && (t >> 4) < REST) store(rest, sum, other);
         }
       } else {
         for (int k = t; k < K; k += T) {
@@ -349,34 +396,47 @@ __device__ __forceinline__ bool layer_setup(const Batch& b, const Work& w, const
         ssp_scat[o + 3 * (size_t)nn * nn + (size_t)row * nn + col] = p1;
       }
     }
-    // ---------------- CHECK_NORM4 (src/radscat4.f90:87-136)
-    if (t < N) {
-      double sum = emis - ext;
-      for (int j2 = 0; j2 < N; j2++)
-        sum = sum + 2.0 * 3.1415926535897932384 * S.wq[j2] * (Tb[(2 * t) * LD + 2 * j2] + Rb[(2 * t) * LD + 2 * j2]);
-      S.nrm[t] = fabs(sum);
-    }
-    team_sync();
-    if (t == 0) {
-      double mx = 0.0;
-      for (int i = 0; i < N; i++) mx = fmax(mx, S.nrm[i]);
-      S.stat = (mx > 5.0e-4) ? (PAMTRA_B200_FATAL | PAMTRA_B200_ST_NORM) : 0;
-    }
-    // ---------------- number of doublings (src/radtran4.f90:319-329)
+    const double planck0 = S.lin[1], planck1 = S.lin[0];
+    // ---------------- number of doublings (src/radtran4.f90:319-329): INT(LOG(tau /
+    // 1e-6) / LN2) + 1.  The logarithm in single precision is good to 1e-4 here; only
+    // next to a whole number does the double-precision one decide.
     const double extinct = ext + gas;
-    const double fl = log(fmax(extinct * zdiff, 1.0e-7) / 1.0e-6) / LN2_F32;
+    const double tau = fmax(extinct * zdiff, 1.0e-7);
     int nd = 0;
-    if (fl > 0.0) nd = (int)fl + 1;
-    const double num_sub = ldexp(1.0, nd);
-    const double delta_z = zdiff / num_sub;
+    {
+      const float flf = log2f((float)(tau * 1.0e6));
+      if (fabsf(flf - rintf(flf)) > 1.0e-3f && flf < 100.0f) {
+        if (flf > 0.0f) nd = (int)flf + 1;
+      } else {
+        const double fl = log(tau / 1.0e-6) / LN2_F32;
+        if (fl > 0.0) nd = (int)fl + 1;
+      }
+    }
+    const double inv_sub = ldexp(1.0, -nd);
+    const double delta_z = zdiff * inv_sub;
+    // ---------------- CHECK_NORM4 (src/radscat4.f90:87-136), eight lanes per angle
+    bool bad;
+    {
+      const int j = t >> 3;
+      double sum = 0.0;
+#pragma unroll
+      for (int j2 = t & 7; j2 < N; j2 += 8)
+        sum = sum + 2.0 * 3.1415926535897932384 * S.wq[j2] * (Tb[(2 * j) * LD + 2 * j2] + Rb[(2 * j) * LD + 2 * j2]);
+#pragma unroll
+      for (int o = 1; o < 8; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+      bad = fabs(emis - ext + sum) > 5.0e-4;
+      if ((t & 7) == 0) S.nrm[j] = delta_z / S.mu[j];
+    }
+    if (__syncthreads_or(bad)) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_NORM;
     // ---------------- INITIALIZE4 (src/radintg4.f90:1-45), in place over P1/P2
     {
       const double C = 2.0 * 3.1415926535897932384;
+#pragma unroll 4
       for (int e = t; e < n * n; e += T) {
         const int col = e / n, row = e % n;
         const int i1 = col & 1, j1 = col >> 1, i2 = row & 1, j2 = row >> 1;
         const double wj1 = S.wq[j1];
-        const double tmp = delta_z / S.mu[j2];
+        const double tmp = S.nrm[j2];
         const double gext = (i1 == i2) ? gas : 0.0;
         const double diag = (row == col) ? 1.0 : 0.0;
         double ex = 0.0;
@@ -395,9 +455,8 @@ __device__ __forceinline__ bool layer_setup(const Batch& b, const Work& w, const
       S.cst[t] = v;
       S.cst[n + t] = v;
     }
-    double linfac = (planck0 == 0.0) ? 0.0 : (planck1 / planck0 - 1.0) / num_sub;
+    double linfac = (planck0 == 0.0) ? 0.0 : (planck1 / planck0 - 1.0) * inv_sub;
     team_sync();
-    status |= S.stat;
   it.c = c;
   it.z = z;
   it.fi = fi;
