@@ -13,7 +13,7 @@
 //   2. the m >= 1 blocks (TMATR, :1765-2047), each one more solve;
 //   3. the T-matrix stored in single precision, as the reference stores it
 //      (REAL*4 common /TMAT/), and the vectors U below.
-// k_tmat_ampl, the amplitude matrices of 30 scattering azimuths for every pair
+// k_tmat_ampl, the amplitude matrices of 16 scattering azimuths (of 30, the others are mirror images) for every pair
 // of Lobatto angles (calc_single_tmatrix, src/tmatrix.f90:436-684): a unit is a
 // scattered angle of a canted particle, or 128 (incident, scattered) pairs of an upright
 // one, so that few particles fill the chip too.
@@ -30,14 +30,14 @@
 // sums of CAL o T with its own Wigner vectors).  U is formed once per
 // incident angle.  For an upright particle (canting 0) the scattered polar
 // angle does not depend on the azimuth: P_m is formed once per scattered angle
-// and the 30 azimuths weigh it; a canted particle forms P_m per scattered
+// and the 16 azimuths weigh it; a canted particle forms P_m per scattered
 // direction, 960 times fewer products than evaluating AMPL per pair.
 // 1024 upright particles of NMAX 5 - 14 (1.2 - 6 mm, 89 GHz): 8.6 ms with one
-// barrier chain per particle and AMPL per pair, now 0.99 ms; 96 canted ones 39 ms,
-// now 0.59 ms.  Bound by latency (pivots, recurrences and phases that follow one
-// another: FP64 pipe 24 % while a CTA is busy).  Four warps per CTA and four
-// CTAs per SM: 1.16 ms upright, 0.74 ms canted; one order after another with a
-// warp per solve: 1.36 ms and 0.72 ms.
+// barrier chain per particle and AMPL per pair, now 0.88 ms; 96 canted ones 39 ms,
+// now 0.43 ms (0.99 and 0.59 ms with all 30 azimuths).  Bound by latency (pivots,
+// recurrences and phases that follow one another: FP64 pipe 24 % while a CTA is
+// busy).  With 30 azimuths, four warps per CTA and four CTAs per SM: 1.16 and
+// 0.74 ms; one order after another with a warp per solve: 1.36 and 0.72 ms.
 // The reference computes the solve in REAL*16; FP64 here agrees with it to
 // about 1e-12 relative on microwave hydrometeors, below the single-precision
 // storage of T.  The normalisation factors the reference forms in
@@ -85,12 +85,20 @@ __device__ __forceinline__ int tm_t0(int nmax, int m) {
   return 4 * (nmax * nmax + tm_cubes(nmax) - tm_cubes(nmax - m + 1));
 }
 // Slot of k_tmatrix: solve pool, T, incident Wigner vectors [pair][2][nummu].
+// Of the TM_NAZ azimuths 12 k degrees only k = 0 .. 15 are formed, k = 1 .. 14 with
+// weight two: mirrored in the plane of the incident direction and the
+// particle's axis, scattered azimuth f at incident azimuth i gives the same
+// forms (F(f, i) = F(-f, -i)).  The reference's 1e-8 offset e of the incident
+// azimuth makes the partner F(-f, e) = F(f, -e), and F(f, e) + F(f, -e) is 2 F(f, 0) to
+// e^2: so these are formed at incident azimuth 0 (1e-14 where 0 is singular).
+constexpr int TM_NAZH = TM_NAZ / 2 + 1;
+static_assert(TM_NAZ % 2 == 0, "a mirrored pair of azimuths each");
 constexpr int TM_DIRD = 7;  // doubles of one direction: polar cosine, cos and sin of the azimuth, rotation
 struct TmSlot {
   size_t t, dvi, total;
 };
 __host__ __device__ inline size_t tm_geo_doubles(int nummu) {
-  return (size_t)TM_DIRD * (2 * (size_t)nummu * TM_NAZ + nummu);
+  return (size_t)TM_DIRD * (2 * (size_t)nummu * TM_NAZH + nummu);
 }
 __host__ __device__ inline TmSlot tm_slot(int nummu) {
   TmSlot s;
@@ -107,8 +115,8 @@ __host__ __device__ inline size_t tm_record(int npair, int nummu, bool upright) 
 }
 // Scratch of a CTA of k_tmat_ampl whose working set exceeds its shared memory.
 constexpr int TMA_SMEM = 9 * 8 * TMA_THREADS;  // doubles: P of an upright particle up to NMAX 8
-constexpr size_t TMA_SLOT = (size_t)TM_PAIRS * 64 > (size_t)(TM_NMAX + 1) * 8 * TMA_THREADS
-                                ? (size_t)TM_PAIRS * 64 : (size_t)(TM_NMAX + 1) * 8 * TMA_THREADS;
+constexpr size_t TMA_SLOT = (size_t)TM_PAIRS * 2 * TM_NAZH > (size_t)(TM_NMAX + 1) * 8 * TMA_THREADS
+                                ? (size_t)TM_PAIRS * 2 * TM_NAZH : (size_t)(TM_NMAX + 1) * 8 * TMA_THREADS;
 
 // ---------------------------------------------------------------- tables of the context
 // Gauss-Legendre nodes and weights of the even orders 2 g, g = 1 .. TM_NGAUSS
@@ -119,7 +127,7 @@ constexpr int TM_SQ = TM_NMAX + 2;
 constexpr size_t TMT_X = 0, TMT_W = TMT_X + (size_t)TM_NGAUSS * (TM_NGAUSS + 1), TMT_CAL = TMT_W + (size_t)TM_NGAUSS * (TM_NGAUSS + 1),
                  TMT_SQ = TMT_CAL + (size_t)TM_NMAX * TM_NMAX, TMT_RQ = TMT_SQ + (size_t)TM_SQ * TM_SQ,
                  TMT_AM = TMT_RQ + (size_t)TM_SQ * TM_SQ, TMT_I2 = TMT_AM + TM_SQ, TMT_CS = TMT_I2 + TM_SQ,
-                 TMT_TOTAL = TMT_CS + (size_t)(TM_NMAX + 1) * TM_NAZ * 2;
+                 TMT_TOTAL = TMT_CS + (size_t)(TM_NMAX + 1) * TM_NAZH * 2;
 
 // Inputs and outputs of one launch: particle p = item * nbins + bin.
 // Counters of a round (all zero at the start, but n): particles, records.  A
@@ -748,7 +756,7 @@ __device__ __forceinline__ void tm_vigampl(double x, int nmax, int m, F&& put) {
 
 // Geometry of AMPL (tmatrix_amplq.lp.f:618-795) for one direction (polar tl,
 // azimuth pl in degrees, with the reference's 1e-8 offsets away from the
-// singular values): the particle-frame polar cosine, the particle-frame
+// singular values; that of the azimuth is epsp): the particle-frame polar cosine, the particle-frame
 // azimuth and the lab -> particle polarisation rotation, inverted for the
 // scattered direction.  The incident and the scattered direction go through
 // the same steps in the reference, so a table of each (per incident angle,
@@ -756,15 +764,15 @@ __device__ __forceinline__ void tm_vigampl(double x, int nmax, int m, F&& put) {
 struct TmDir {
   double ctp, phip, M[2][2];
 };
-__device__ void tm_dir(double tl, double pl, double alpha, double beta, bool invert, TmDir& d) {
+__device__ void tm_dir(double tl, double pl, double alpha, double beta, bool invert, double epsp, TmDir& d) {
   const double pin = 3.141592653589793, pin2 = pin * 0.5, pi = pin / 180.0;
   const double alph = alpha * pi;
   double bet = beta * pi, thetl = tl * pi, phil = pl * pi;
   const double eps = 1e-8;
   if (thetl < pin2) thetl = thetl + eps;
   if (thetl > pin2) thetl = thetl - eps;
-  if (phil < pin) phil = phil + eps;
-  if (phil > pin) phil = phil - eps;
+  if (phil < pin) phil = phil + epsp;
+  if (phil > pin) phil = phil - epsp;
   if (bet <= pin2 && pin2 - bet <= eps) bet = bet - eps;
   if (bet > pin2 && bet - pin2 <= eps) bet = bet + eps;
   const double cb = cos(bet), sb = sin(bet);
@@ -848,9 +856,9 @@ __global__ void __launch_bounds__(TM_NGAUSS) k_tmat_tables(double* tab) {
 
 // Directions of a particle of canting angle beta as [TM_DIRD][azimuth][angle]
 // (scattered, inverted rotations), then [TM_DIRD][incident angle]: element e
-// of 2 nummu TM_NAZ + nummu.
+// of 2 nummu TM_NAZH + nummu.
 __device__ __forceinline__ void tm_geo(double* geo, int nummu, const double* mu, double beta, int e) {
-  const int na = 2 * nummu, ns = na * TM_NAZ;
+  const int na = 2 * nummu, ns = na * TM_NAZH;
   TmDir d;
   double* o;
   int stride;
@@ -859,13 +867,13 @@ __device__ __forceinline__ void tm_geo(double* geo, int nummu, const double* mu,
     double th = acos(mu[ll] * (kk == 0 ? 1.0 : -1.0)) * 180.0 / PI;
     if (th > 179.9999) th = 180.0;
     const double phi = 360.0 / (double)TM_NAZ * ((double)(k + 1) - 1.0);
-    tm_dir(th, phi, 0.0, beta, true, d);
+    tm_dir(th, phi, 0.0, beta, true, 1e-8, d);
     o = geo + e;
     stride = ns;
   } else {
     double th0 = acos(mu[e - ns] * 1.0) * 180.0 / PI;
     if (th0 > 179.9999) th0 = 180.0;
-    tm_dir(th0, 0.0, 0.0, beta, false, d);
+    tm_dir(th0, 0.0, 0.0, beta, false, beta == 0.0 ? 1e-8 : 1e-14, d);
     o = geo + TM_DIRD * ns + (e - ns);
     stride = nummu;
   }
@@ -881,20 +889,21 @@ __device__ __forceinline__ void tm_geo(double* geo, int nummu, const double* mu,
 }
 __global__ void k_tmat_geo(double* geo, int nummu, const double* mu) {
   const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e < 2 * nummu * TM_NAZ + nummu) tm_geo(geo, nummu, mu, 0.0, e);
+  if (e < 2 * nummu * TM_NAZH + nummu) tm_geo(geo, nummu, mu, 0.0, e);
 }
 // TMT_CS: the azimuth difference of an upright particle depends on neither
 // polar angle; angle-addition recurrence
 __global__ void k_tmat_azimuth(double* tab, const double* geo, int nummu) {
-  const int t = threadIdx.x, na = 2 * nummu, ns = na * TM_NAZ;
-  if (t >= TM_NAZ) return;
+  const int t = threadIdx.x, na = 2 * nummu, ns = na * TM_NAZH;
+  if (t >= TM_NAZH) return;
   const double* gin = geo + TM_DIRD * ns;
-  const double cs = geo[ns + t * na], ss = geo[2 * ns + t * na], ci = gin[nummu], si = gin[2 * nummu];
+  const bool pair = t > 0 && t < TM_NAZH - 1;
+  const double cs = geo[ns + t * na], ss = geo[2 * ns + t * na], ci = pair ? 1.0 : gin[nummu], si = pair ? 0.0 : gin[2 * nummu];
   const double c1 = fma(cs, ci, ss * si), s1 = fma(ss, ci, -cs * si);
   double cm = 1.0, sm = 0.0;
   for (int m = 0; m <= TM_NMAX; m++) {
-    tab[TMT_CS + (m * TM_NAZ + t) * 2] = m ? 2.0 * cm : 1.0;
-    tab[TMT_CS + (m * TM_NAZ + t) * 2 + 1] = 2.0 * sm;
+    tab[TMT_CS + (m * TM_NAZH + t) * 2] = m ? 2.0 * cm : 1.0;
+    tab[TMT_CS + (m * TM_NAZH + t) * 2 + 1] = 2.0 * sm;
     const double cn = cm * c1 - sm * s1;
     sm = sm * c1 + cm * s1;
     cm = cn;
@@ -1026,30 +1035,30 @@ struct TmUnit {
   }
 };
 
-// Scattered angle a of a canted particle: the Wigner vectors of its 30
+// Scattered angle a of a canted particle: the Wigner vectors of its 16
 // azimuths, then (incident angle, two azimuths) per thread.  buf: DV
-// [pair][2][32] where it fits shared memory, then the azimuth terms.
+// [pair][2][azimuth] where it fits shared memory, then the azimuth terms.
 __device__ __forceinline__ void tm_canted(const TmArgs& A, const TmUnit& X, int a, double* buf, double* scratch) {
   constexpr int KB = 2;
-  const int t = threadIdx.x, nummu = A.nummu, na = 2 * nummu, ns = na * TM_NAZ, nmax = X.nmax;
+  const int t = threadIdx.x, nummu = A.nummu, na = 2 * nummu, ns = na * TM_NAZH, nmax = X.nmax;
   const int npair = tm_pair0(nmax, nmax) + 1;
   const double *U = X.rec, *geo = U + (size_t)npair * 8 * nummu, *gin = geo + TM_DIRD * ns;
   double* const zt = buf;  // [azimuth][4][nummu]
-  double* const DV = TM_NAZ * 4 * nummu + npair * 64 <= TMA_SMEM ? buf + TM_NAZ * 4 * nummu : scratch;
+  double* const DV = TM_NAZH * 4 * nummu + npair * 2 * TM_NAZH <= TMA_SMEM ? buf + TM_NAZH * 4 * nummu : scratch;
   const double phi_weights = 1.0 / 360.0 * (360.0 / TM_NAZ);
-  for (int e = t; e < (nmax + 1) * TM_NAZ; e += TMA_THREADS) {
-    const int m = e / TM_NAZ, k = e % TM_NAZ;
-    tm_wigner(geo[k * na + a], nmax, m, A.tab, DV + tm_pair0(nmax, m) * 64 + k, 32);
+  for (int e = t; e < (nmax + 1) * TM_NAZH; e += TMA_THREADS) {
+    const int m = e / TM_NAZH, k = e % TM_NAZH;
+    tm_wigner(geo[k * na + a], nmax, m, A.tab, DV + tm_pair0(nmax, m) * 2 * TM_NAZH + k, TM_NAZH);
   }
   __syncthreads();
   const int jj = t % nummu, slot = t / nummu, nslot = TMA_THREADS / nummu;
   const double ci = gin[nummu + jj], si = gin[2 * nummu + jj];
-  for (int k0 = slot * KB; k0 < TM_NAZ; k0 += nslot * KB) {
+  for (int k0 = slot * KB; k0 < TM_NAZH; k0 += nslot * KB) {
     int k[KB];
     double amp[KB][8], c1[KB], s1[KB], cm[KB], sm[KB];
 #pragma unroll
     for (int j = 0; j < KB; j++) {
-      k[j] = min(k0 + j, TM_NAZ - 1);
+      k[j] = min(k0 + j, TM_NAZH - 1);
       // azimuth difference of the scattered and the incident direction
       const double cs = geo[ns + k[j] * na + a], ss = geo[2 * ns + k[j] * na + a];
       c1[j] = fma(cs, ci, ss * si);
@@ -1063,8 +1072,8 @@ __device__ __forceinline__ void tm_canted(const TmArgs& A, const TmUnit& X, int 
     for (int m = 0; m <= nmax; m++) {
       const int nm = nmax - max(m, 1) + 1;
       double x[KB][8];
-      tm_pm<KB>(d, 32, k, u, nummu, nm, x);
-      d += nm * 64;
+      tm_pm<KB>(d, TM_NAZH, k, u, nummu, nm, x);
+      d += nm * 2 * TM_NAZH;
       u += nm * 8 * nummu;
 #pragma unroll
       for (int j = 0; j < KB; j++) {
@@ -1083,7 +1092,7 @@ __device__ __forceinline__ void tm_canted(const TmArgs& A, const TmUnit& X, int 
     }
 #pragma unroll
     for (int j = 0; j < KB; j++) {
-      if (k0 + j >= TM_NAZ) continue;
+      if (k0 + j >= TM_NAZH) continue;
       double z[4];
       tm_forms(amp[j], gin + 3 * nummu + jj, nummu, geo + 3 * ns + k[j] * na + a, ns, X.fact, z);
       if (k[j] == 0) {
@@ -1091,26 +1100,27 @@ __device__ __forceinline__ void tm_canted(const TmArgs& A, const TmUnit& X, int 
         if (a == jj) tm_forward(X.ext, jj, X.fext, amp[j]);
       }
 #pragma unroll
-      for (int c = 0; c < 4; c++) zt[(k[j] * 4 + c) * nummu + jj] = z[c] * phi_weights;
+      for (int c = 0; c < 4; c++)
+        zt[(k[j] * 4 + c) * nummu + jj] = z[c] * (k[j] == 0 || k[j] == TM_NAZH - 1 ? phi_weights : 2.0 * phi_weights);
     }
   }
   __syncthreads();
   for (int e = t; e < 4 * nummu; e += TMA_THREADS) {
     double z = 0.0;
-#pragma unroll 10
-    for (int k = 0; k < TM_NAZ; k++) z = z + zt[k * 4 * nummu + e];
+#pragma unroll 8
+    for (int k = 0; k < TM_NAZH; k++) z = z + zt[k * 4 * nummu + e];
     const int c = e / nummu, j = e % nummu, kk = a / nummu, ll = a % nummu;
     X.scat[(c >> 1) + 2 * (ll + nummu * ((c & 1) + 2 * (j + nummu * kk)))] = z;
   }
 }
 
 // 128 (incident, scattered) angle pairs of an upright particle, one per
-// thread: P_m of every order into the thread's own column of buf, then the 30 azimuths, five
+// thread: P_m of every order into the thread's own column of buf, then the 16 azimuths, four
 // at a time.  No barrier.
 __device__ __forceinline__ void tm_upright(const TmArgs& A, const TmUnit& X, int part, double* buf, double* scratch) {
-  constexpr int KB = 5;
-  static_assert(TM_NAZ % KB == 0, "azimuths per pass");
-  const int t = threadIdx.x, nummu = A.nummu, na = 2 * nummu, ns = na * TM_NAZ, nmax = X.nmax;
+  constexpr int KB = 4;
+  static_assert(TM_NAZH % KB == 0, "azimuths per pass");
+  const int t = threadIdx.x, nummu = A.nummu, na = 2 * nummu, ns = na * TM_NAZH, nmax = X.nmax;
   const int npair = tm_pair0(nmax, nmax) + 1;
   const int a = t % na, jj = part * (TMA_THREADS / na) + t / na;
   double* const P = ((nmax + 1) * 8 * TMA_THREADS <= TMA_SMEM ? buf : scratch) + t;
@@ -1137,7 +1147,7 @@ __device__ __forceinline__ void tm_upright(const TmArgs& A, const TmUnit& X, int
   const double *geo = A.geo, *gin = geo + TM_DIRD * ns, *cst = A.tab + TMT_CS;
   const double phi_weights = 1.0 / 360.0 * (360.0 / TM_NAZ);
   double zs[4] = {0.0, 0.0, 0.0, 0.0};
-  for (int k0 = 0; k0 < TM_NAZ; k0 += KB) {
+  for (int k0 = 0; k0 < TM_NAZH; k0 += KB) {
     double amp[KB][8];
 #pragma unroll
     for (int j = 0; j < KB; j++)
@@ -1149,7 +1159,7 @@ __device__ __forceinline__ void tm_upright(const TmArgs& A, const TmUnit& X, int
       for (int c = 0; c < 8; c++) x[c] = P[(m * 8 + c) * TMA_THREADS];
 #pragma unroll
       for (int j = 0; j < KB; j++) {
-        const double2 cs = *reinterpret_cast<const double2*>(cst + (m * TM_NAZ + k0 + j) * 2);
+        const double2 cs = *reinterpret_cast<const double2*>(cst + (m * TM_NAZH + k0 + j) * 2);
 #pragma unroll
         for (int e = 0; e < 2; e++) {
           amp[j][e] = fma(cs.x, x[e], amp[j][e]);
@@ -1169,7 +1179,7 @@ __device__ __forceinline__ void tm_upright(const TmArgs& A, const TmUnit& X, int
         if (a == jj) tm_forward(X.ext, jj, X.fext, amp[j]);
       }
 #pragma unroll
-      for (int c = 0; c < 4; c++) zs[c] = zs[c] + z[c] * phi_weights;
+      for (int c = 0; c < 4; c++) zs[c] = zs[c] + z[c] * (k == 0 || k == TM_NAZH - 1 ? phi_weights : 2.0 * phi_weights);
     }
   }
   const int kk = a / nummu, ll = a % nummu;
@@ -1367,7 +1377,7 @@ __device__ void tm_particle(const TmArgs& A, double* s, const TmSlot& L, TmShare
   double* const U = A.records + sh.rec;
   double* const rest = U + (size_t)npair * 8 * nummu;  // scattered Wigner vectors or directions
   double* const DVI = s + L.dvi;
-  const int ns = na * TM_NAZ;
+  const int ns = na * TM_NAZH;
   const double* geo = A.geo;
   if (!upright) {
     for (int e = t; e < ns + nummu; e += TM_THREADS) tm_geo(rest, nummu, A.mu, beta, e);

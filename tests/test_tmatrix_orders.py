@@ -38,6 +38,19 @@ def test_gpu_tmatrix_orders(oracle_mod, x, asr, nummu):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("node", [0, 4, 7])
+def test_gpu_tmatrix_axis_along_an_angle(oracle_mod, node):
+    """A canted particle whose axis is one of the incident directions (a Lobatto
+    node, the last one 0 deg): the particle frame's azimuth is singular there."""
+    leg = np.polynomial.legendre.Legendre.basis(15).deriv().roots()  # Gauss-Lobatto rule of 16 points
+    mu = np.append(np.sort(leg[leg > 0]), 1.0)[node]
+    beta = float(np.degrees(np.arccos(mu)))
+    items = [_ice((0.5, 2.0), 0.6, b) for b in (beta, 180.0 - beta)]
+    out = _run_gpu(items, 3, 8)
+    _compare(out, [_oracle_item(oracle_mod, it, 8) for it in items], 8)
+
+
+@pytest.mark.gpu
 def test_gpu_tmatrix_record_rounds(oracle_mod):
     """More particles than one round of records holds (about 2800 of each kind
     here), upright and canted in turn, some invalid: equal particles give
