@@ -470,6 +470,7 @@ struct pamtra_b200_ctx {
   size_t tm_bytes = 0;
   char* stage = nullptr;  // device staging for run_host
   size_t stage_bytes = 0;
+  char* pin = nullptr;  // pinned staging of small run_host calls: inputs, then outputs (HOST_PIN bytes each)
   // launch shapes (pamtra_b200_set_launch; 0 = occupancy default)
   int mie_warps = MIE_WARPS;  // warps per k_mie CTA (2, 4 or 8)
   int mie_cps = 0;            // k_mie CTAs per SM
@@ -612,6 +613,7 @@ int32_t pamtra_b200_destroy(pamtra_b200_ctx* ctx) {
   cudaFree(ctx->mie_tab);
   cudaFree(ctx->lob_mu);
   cudaFree(ctx->lob_w);
+  cudaFreeHost(ctx->pin);
   cudaFree(ctx->stage);
   cudaFree(ctx->tm_buf);
   cudaFree(ctx->tm_tab);
@@ -1037,6 +1039,8 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   return cudaGetLastError() == cudaSuccess ? PAMTRA_B200_OK : PAMTRA_B200_FATAL;
 }
 
+constexpr size_t HOST_PIN = (size_t)256 << 10;
+
 int32_t pamtra_b200_run_host(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, const pamtra_b200_columns* hc,
                              const pamtra_b200_outputs* ho, int32_t precision, void* stream_) {
   if (!ctx || !st || !hc || !ho || !ho->tb) return PAMTRA_B200_FATAL;
@@ -1096,7 +1100,21 @@ int32_t pamtra_b200_run_host(pamtra_b200_ctx* ctx, const pamtra_b200_settings* s
     ctx->stage_bytes = off + off / 8;
   }
   char* D = ctx->stage;
-  for (auto& s : in) cudaMemcpyAsync(D + s.off, s.h, s.bytes, cudaMemcpyHostToDevice, stream);
+  // Small calls gather their inputs in pinned memory and copy once, and read
+  // their outputs back in one copy: a pageable copy costs a few microseconds
+  // whatever its size, and a column has eighteen inputs and up to eighteen outputs (one
+  // column 0.93 -> 0.83 ms).  Larger ones pay more for the gathering than for the calls.
+  const bool pin_in = o_tb <= HOST_PIN, pin_out = off - o_tb <= HOST_PIN;
+  if ((pin_in || pin_out) && !ctx->pin && cudaMallocHost(&ctx->pin, 2 * HOST_PIN) != cudaSuccess) {
+    ctx->pin = nullptr;
+    return PAMTRA_B200_FATAL;
+  }
+  if (pin_in) {
+    for (auto& s : in) memcpy(ctx->pin + s.off, s.h, s.bytes);
+    cudaMemcpyAsync(D, ctx->pin, o_tb, cudaMemcpyHostToDevice, stream);
+  } else {
+    for (auto& s : in) cudaMemcpyAsync(D + s.off, s.h, s.bytes, cudaMemcpyHostToDevice, stream);
+  }
   pamtra_b200_columns dc = *hc;
   auto dp = [&](const void* h, size_t o) -> const void* { return h ? (const void*)(D + o) : nullptr; };
   dc.nlyrs = (const int32_t*)dp(hc->nlyrs, o_nly);
@@ -1148,28 +1166,41 @@ int32_t pamtra_b200_run_host(pamtra_b200_ctx* ctx, const pamtra_b200_settings* s
   }
   if (dout.scatter_matrix) cudaMemsetAsync(dout.scatter_matrix, 0, C * Fm * Lm * 4 * NA * NA * 8, stream);
   int32_t rc = pamtra_b200_run(ctx, st, &dc, &dout, precision, stream);
-  if (rc != PAMTRA_B200_OK) return rc;
-  cudaMemcpyAsync(ho->tb, dout.tb, C * NO * NA * Fm * 2 * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->emissivity) cudaMemcpyAsync(ho->emissivity, dout.emissivity, C * 2 * Fm * hc->max_nummu * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->angles_deg) cudaMemcpyAsync(ho->angles_deg, dout.angles_deg, NA * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->status) cudaMemcpyAsync(ho->status, dout.status, C * Fm * 4, cudaMemcpyDeviceToHost, stream);
-  if (ho->kextatmo) cudaMemcpyAsync(ho->kextatmo, dout.kextatmo, C * Fm * Lm * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->kexttot) cudaMemcpyAsync(ho->kexttot, dout.kexttot, C * Fm * Lm * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->salbedo) cudaMemcpyAsync(ho->salbedo, dout.salbedo, C * Fm * Lm * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->scatter_matrix)
-    cudaMemcpyAsync(ho->scatter_matrix, dout.scatter_matrix, C * Fm * Lm * 4 * NA * NA * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->num_doubles) cudaMemcpyAsync(ho->num_doubles, dout.num_doubles, C * Fm * Lm * 4, cudaMemcpyDeviceToHost, stream);
-  if (ho->ze) cudaMemcpyAsync(ho->ze, dout.ze, C * Fm * Lm * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->att_hydro) cudaMemcpyAsync(ho->att_hydro, dout.att_hydro, C * Fm * Lm * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->att_atmo) cudaMemcpyAsync(ho->att_atmo, dout.att_atmo, C * Fm * Lm * 8, cudaMemcpyDeviceToHost, stream);
-  if (ho->psd_d) {
-    cudaMemcpyAsync(ho->psd_d, dout.psd_d, NP * 8, cudaMemcpyDeviceToHost, stream);
-    cudaMemcpyAsync(ho->psd_deltad, dout.psd_deltad, NP * 8, cudaMemcpyDeviceToHost, stream);
-    cudaMemcpyAsync(ho->psd_n, dout.psd_n, NP * 8, cudaMemcpyDeviceToHost, stream);
-    cudaMemcpyAsync(ho->psd_mass, dout.psd_mass, NP * 8, cudaMemcpyDeviceToHost, stream);
-    cudaMemcpyAsync(ho->psd_area, dout.psd_area, NP * 8, cudaMemcpyDeviceToHost, stream);
-    cudaMemcpyAsync(ho->psd_bscat, dout.psd_bscat, NP * 8, cudaMemcpyDeviceToHost, stream);
+  if (rc != PAMTRA_B200_OK) {
+    cudaStreamSynchronize(stream);  // the pinned inputs may be on their way
+    return rc;
   }
+  struct OutSeg { void* h; size_t off, bytes; };
+  std::vector<OutSeg> res;
+  auto get = [&](void* h, const void* d, size_t bytes) { if (h) res.push_back({h, (size_t)((const char*)d - D), bytes}); };
+  get(ho->tb, dout.tb, C * NO * NA * Fm * 2 * 8);
+  get(ho->emissivity, dout.emissivity, C * 2 * Fm * hc->max_nummu * 8);
+  get(ho->angles_deg, dout.angles_deg, NA * 8);
+  get(ho->status, dout.status, C * Fm * 4);
+  get(ho->kextatmo, dout.kextatmo, C * Fm * Lm * 8);
+  get(ho->kexttot, dout.kexttot, C * Fm * Lm * 8);
+  get(ho->salbedo, dout.salbedo, C * Fm * Lm * 8);
+  get(ho->scatter_matrix, dout.scatter_matrix, C * Fm * Lm * 4 * NA * NA * 8);
+  get(ho->num_doubles, dout.num_doubles, C * Fm * Lm * 4);
+  get(ho->ze, dout.ze, C * Fm * Lm * 8);
+  get(ho->att_hydro, dout.att_hydro, C * Fm * Lm * 8);
+  get(ho->att_atmo, dout.att_atmo, C * Fm * Lm * 8);
+  if (ho->psd_d) {
+    get(ho->psd_d, dout.psd_d, NP * 8);
+    get(ho->psd_deltad, dout.psd_deltad, NP * 8);
+    get(ho->psd_n, dout.psd_n, NP * 8);
+    get(ho->psd_mass, dout.psd_mass, NP * 8);
+    get(ho->psd_area, dout.psd_area, NP * 8);
+    get(ho->psd_bscat, dout.psd_bscat, NP * 8);
+  }
+  if (pin_out) {
+    char* const back = ctx->pin + HOST_PIN;
+    cudaMemcpyAsync(back, D + o_tb, off - o_tb, cudaMemcpyDeviceToHost, stream);
+    if (cudaStreamSynchronize(stream) != cudaSuccess) return PAMTRA_B200_FATAL;
+    for (auto& r : res) memcpy(r.h, back + (r.off - o_tb), r.bytes);
+    return PAMTRA_B200_OK;
+  }
+  for (auto& r : res) cudaMemcpyAsync(r.h, D + r.off, r.bytes, cudaMemcpyDeviceToHost, stream);
   if (cudaStreamSynchronize(stream) != cudaSuccess) return PAMTRA_B200_FATAL;
   return PAMTRA_B200_OK;
 }
