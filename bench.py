@@ -9,14 +9,13 @@ layers over 0-12 km, cloud liquid (exp, 40 bins) and rain (Marshall-Palmer,
 50 bins) in layers 5-25 with mixing ratios log-uniform over 0.01-2 g/kg,
 frequencies 23.8, 31.4, 89 and 150 GHz, NUMMU = 16, FP64.
 
-  value  : batched FP64 form (PREC_FP64_BATCHED: one inverse per adding
-           combine) in solves/s with inputs resident in HBM (device-timed,
+  value  : batched FP64 form (PREC_FP64_BATCHED) in solves/s with inputs resident in HBM (device-timed,
            CUDA events on the launching stream, L2 flushed between steps),
            launch shapes from the autotuner
   e2e    : same metric through the C ABI with host buffers (pinned), the
            host<->device copies inside the timed region
-  plain  : the plain form (one column per call, the reference operation
-           order PREC_FP64) on a sample of columns
+  plain  : the plain form (one column per call, PREC_FP64: the same
+           kernels) on a sample of columns
   split_3xtf32 / target_shape / serving / graph_replay: the split-precision
            form, the 150-layer 4-species shape, the request loop and the
            CUDA-graph replay of the same step
@@ -403,8 +402,7 @@ def _target_shape(args, local, eng, stream):
             "tb_err_3xtf32_vs_fp64_K": split_err, "stage_ms_3xtf32": sstages,
             "unit": "solves/s", "batched_ms_per_step": float(np.mean(ms)), "status_nonzero": st_bad,
             "plain_sample_columns": 16, "plain_vs_batched_fp64_tb_max_diff_K": plain_diff,
-            "forms": "batched FP64: one-inverse adding (PREC_FP64_BATCHED); plain: one column per call in the "
-                     "reference operation order (PREC_FP64)"}
+            "forms": "batched FP64 (PREC_FP64_BATCHED); plain: one column per call (PREC_FP64, the same kernels)"}
 
 
 def _config_line(name, b, local, eng, stream, pool, nplain=8, reps=1, noracle=8):
@@ -854,8 +852,8 @@ def main():
                 "flops_per_launch": flops, "kernel_ms": t_layer * 1e3,
                 "achieved_executed": 2.0 * 32 ** 3 * layer_products / t_layer / 1e12 if t_layer > 0 else None,
                 "executed_products_per_launch": layer_products,
-                "executed_note": "n x n products the kernel issued (5 per doubling plus the Neumann/Horner "
-                                 "series, Gauss-Jordan counted as one), 2 n^3 FLOP each, n = 32; the algorithmic "
+                "executed_note": "n x n products the kernel issued (a symmetric one counts its computed tiles; the "
+                                 "series with them, Gauss-Jordan as one), 2 n^3 FLOP each, n = 32; the algorithmic "
                                  "figure counts 6 products and one inverse per doubling"}
     roofline["frac_executed"] = roofline["achieved_executed"] / peak if peak and roofline["achieved_executed"] \
         else None
@@ -892,9 +890,9 @@ def main():
         "cpu_baseline": cpu,
         "clocks": clocks,
         "plain_fp64": {"value": plain_value, "unit": "solves/s",
-                       "form": "one column per call, FP64 in the reference operation order (PREC_FP64)",
+                       "form": "one column per call, FP64 (PREC_FP64)",
                        "tb_max_diff_vs_batched_K": plain_diff},
-        "batched_form": "FP64, one-inverse adding combine (PREC_FP64_BATCHED)",
+        "batched_form": "FP64 (PREC_FP64_BATCHED)",
         "graph_replay": {"value": graph_value, "unit": "solves/s", "ms_per_step": float(np.mean(g_ms)),
                          "tb_equals_direct": graph_same,
                          "form": "the batched FP64 step captured once as a CUDA graph and replayed"},
