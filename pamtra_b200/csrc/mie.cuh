@@ -568,7 +568,7 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
       const int nterms = mie_nstop(xmax);
       int nlegen = min(MAXNLEG - 1, 2 * nterms);
       const int nquad = (nlegen + 2 * nterms + 2) / 2;
-      if (nquad > NQ_MAX || nquad > w.gq_max || nterms + 1 > NT_MAX) {
+      if (nquad > NQ_MAX || nquad > w.gq_max || nterms < 0 || nterms >= NT_MAX) {
         status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;
         break;
       }
@@ -588,7 +588,7 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
       }
 #pragma unroll
       for (int o = 16; o > 0; o >>= 1) dmax = fmax(dmax, __shfl_xor_sync(0xffffffffu, dmax, o));
-      int kmax = max(nterms, dmax > diaN ? min(mie_nstop(PI * dmax / wl) + 1, NT_MAX - 1) : min(nterms + 1, NT_MAX - 1));
+      int kmax = max(nterms, min(dmax > diaN ? mie_nstop(PI * dmax / wl) : nterms, NT_MAX - 2) + 1);
       kmax = (kmax + 3) & ~3;  // terms go in fours
       // bins per pass, a multiple of a group's eight so that no group runs past the slab's columns
       const int bp = min(32, MIE_SLAB / (4 * kmax)) & ~7;
@@ -612,7 +612,7 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
               const cplx ms = (sp_liq_ice == -1 && rho != 917.0) ? eps_mix_m(m_ice, rho) : m_ice;
               const double x = PI * dia / wl;
               int nmie = mie_nstop(x);
-              if (nmie + 1 > NT_MAX) { nmie = NT_MAX - 1; status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE; }
+              if (nmie >= NT_MAX) { nmie = NT_MAX - 1; status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE; }
               double qe, qs, qb;
               miecalc_slab(nmie, x, ms, col, ldc, qe, qs, qb);
               const double r2 = (dia / 2.0) * (dia / 2.0);
