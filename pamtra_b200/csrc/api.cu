@@ -953,7 +953,9 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
     const int mw = ctx->mie_warps;
     const size_t sm_mie = mw * sizeof(MieSmem);
     const void* kmie = ctx->mie_group == 8 ? (const void*)k_mie<2> : (const void*)k_mie<1>;
-    int g = std::min(persistent_grid(kmie, 32 * mw, sm_mie, sms, ctx->mie_cps), std::max(1, pl.mie_nslab / mw));
+    // CTAs for every slab: rounded down, the 63 items of one column (21 layers x 3 frequencies)
+    // had 60 warps, and three items waited for another to end (k_mie 87 us, with 16 CTAs 54 us)
+    int g = std::min(persistent_grid(kmie, 32 * mw, sm_mie, sms, ctx->mie_cps), std::max(1, (pl.mie_nslab + mw - 1) / mw));
     const size_t nref = (size_t)std::max(1, pl.pmax) * Fm;
     k_refr<<<(unsigned)((nref + 127) / 128), 128, 0, stream>>>(b, w, *st); launches++;
     if (ctx->mie_group == 8) k_mie<2><<<g, 32 * mw, sm_mie, stream>>>(b, w, *st);

@@ -77,3 +77,31 @@ def test_phase_matrices_of_even_and_odd_series(oracle_mod, native, nummu):
         assert ssp._compare(one, out, oracle_mod, nummu) >= 1
         passed += 1
     assert passed >= 5
+
+
+@pytest.mark.parametrize("nlay,nfreq", [(1, 1), (3, 1), (3, 3), (7, 9)])
+def test_items_around_the_warps_of_a_cta(native, nlay, nfreq):
+    """1, 3, 9 and 63 items in CTAs of 2, 4 and 8 warps: the last CTA is partly
+    idle.  Items do not depend on one another, so the bytes are the same."""
+    import torch
+    b = _batch((8, 9, 16, 8), nlay=max(nlay, 2))
+    q = b.host["hydro_q"]
+    q[:, nlay:] = 0.0
+    one = pbatch.pack_columns(b.settings, b.species, dict(b.host, freqs=np.array(FREQS[:nfreq]), max_nfreq=nfreq),
+                              b.species_stride)
+    eng = native.engine(0)
+    keep = eng.get_launch()
+    outs = []
+    try:
+        for warps in (2, 4, 8):
+            eng.set_launch((warps, 0, 0, 0, 4))
+            out = ssp._outputs(one, torch.device("cuda", 0))
+            pbatch.run(one, 0, out)
+            torch.cuda.synchronize()
+            outs.append({k: out[k].clone() for k in ("kexttot", "salbedo", "scatter_matrix", "tb", "status")})
+    finally:
+        eng.set_launch(keep)
+    assert int((outs[0]["kexttot"] > 0).sum()) == nlay * nfreq
+    for o in outs[1:]:
+        for k, v in o.items():
+            assert np.array_equal(v.cpu().numpy(), outs[0][k].cpu().numpy(), equal_nan=True), (k, nlay, nfreq)
