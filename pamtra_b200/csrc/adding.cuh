@@ -532,7 +532,7 @@ struct Adder {
                                                 const pamtra_b200_outputs& out, SM& S, const RG& G, int i, int c,
                                                 int fi, bool scat, int status) {
     const int t = threadIdx.x, lane = t & 31, g = lane >> 2, q = lane & 3, row = 8 * i + g;
-    const int Fm = b.max_nfreq, L = b.nlyrs[c];
+    const int Fm = b.max_nfreq, L = b.layers(c);
     const double wl = C_LIGHT / (b.freq(c, fi) * 1.e3);
     const char refl = (char)b.sfc_refl[c];
     const double e = st.emissivity, rr = 1.0 - e;
@@ -629,10 +629,17 @@ struct Adder {
         tbo[dn_i + 1] = rad_to_tb(d1, wl);
       }
     }
-    if (out.emissivity)
-      for (int k = t; k < 2 * N; k += T)
-        out.emissivity[(((size_t)c * 2 + k / N) * Fm + fi) * b.max_nummu + k % N] = e;
+    put_emissivity(b, st, out, c, fi);
     if (t == 0 && status) atomicOr(&w.status[(size_t)c * Fm + fi], status);
+  }
+
+  // The emissivity output of a unit.  Also that of a column whose number of layers is
+  // refused: no radiance is computed for it (tb stays -9999, the status says so).
+  __device__ static __forceinline__ void put_emissivity(const Batch& b, const pamtra_b200_settings& st,
+                                                        const pamtra_b200_outputs& out, int c, int fi) {
+    if (!out.emissivity) return;
+    for (int k = threadIdx.x; k < 2 * N; k += T)
+      out.emissivity[(((size_t)c * 2 + k / N) * b.max_nfreq + fi) * b.max_nummu + k % N] = st.emissivity;
   }
 
   // quadrature nodes and the scaling of the stack's rows (1 when not SYM)
@@ -667,7 +674,11 @@ __global__ void __launch_bounds__(SymTeam<2 * N>::T, (N == 32 ? 1 : 4)) k_adding
     if (item >= nitems) break;
     const int unit = item / maxseg, seg = item % maxseg, c = unit / Fm, fi = unit % Fm;
     if (fi >= b.col_nfreq(c) || b.col_nummu(c) != N) continue;
-    const int L = b.nlyrs[c];
+    const int L = b.layers(c);
+    if (L == 0) {
+      if (seg == 0) A::put_emissivity(b, st, out, c, fi);
+      continue;
+    }
     const int* pres = w.pres_idx + (size_t)c * Lm;
     // scattering layers of the unit, and of this segment: top-down layers k0 .. k1 - 1
     int M = 0;

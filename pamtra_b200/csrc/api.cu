@@ -170,7 +170,7 @@ __global__ void k_ssp_out(Batch b, Work w, pamtra_b200_outputs out) {
   const int Lm = b.max_nlyrs, Fm = b.max_nfreq;
   if (idx >= (size_t)b.ncol * Fm * Lm) return;
   const int z = idx % Lm, f = (idx / Lm) % Fm, c = idx / ((size_t)Lm * Fm);
-  const int p = (z < b.nlyrs[c]) ? w.pres_idx[(size_t)c * Lm + z] : -1;
+  const int p = (z < b.layers(c)) ? w.pres_idx[(size_t)c * Lm + z] : -1;
   const size_t item = (size_t)p * Fm + f;
   if (out.kexttot) out.kexttot[idx] = (p >= 0) ? w.m_kext[item] : 0.0;
   if (out.salbedo) out.salbedo[idx] = (p >= 0) ? w.m_salb[item] : 0.0;
@@ -189,7 +189,7 @@ __global__ void k_radar(Batch b, Work w, pamtra_b200_settings st, pamtra_b200_ou
   if (u >= b.ncol * Fm) return;
   const int c = u / Fm, f = u % Fm;
   const size_t o = ((size_t)c * Fm + f) * Lm;
-  const int L = (f < b.col_nfreq(c)) ? b.nlyrs[c] : 0;
+  const int L = (f < b.col_nfreq(c)) ? b.layers(c) : 0;
   for (int z = 0; z < Lm; z++) {
     if (out.ze) out.ze[o + z] = -9999.0;
     if (out.att_hydro) out.att_hydro[o + z] = 0.0;

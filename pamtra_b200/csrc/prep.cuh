@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(256) k_gas(Batch b, Work w, int lgas, int gas_
   const int f = (idx / Lm) % Fm;
   const int c = idx / ((size_t)Lm * Fm);
   double k = 0.0;
-  if (z < b.nlyrs[c] && f < b.col_nfreq(c) && lgas) {
+  if (z < b.layers(c) && f < b.col_nfreq(c) && lgas) {
     const size_t lz = (size_t)c * Lm + z;
     if (G == 1 && gas_mod == PAMTRA_B200_GAS_L93) {
       k = gas_l93(b.freq(c, f), w.press[lz], w.vap[lz], w.temp[lz]);
@@ -708,7 +708,7 @@ __global__ void __launch_bounds__(32 * PSD_WARPS) k_psd(Batch b, Work w, pamtra_
   auto done = [&](int state, int nbin) {
     if (lane == 0) { w.slot_st[s_idx] = (int8_t)state; w.slot_nb[s_idx] = nbin; }
   };
-  if (z >= b.nlyrs[c]) { done(0, 0); return; }
+  if (z >= b.layers(c)) { done(0, 0); return; }
   const pamtra_b200_species s = b.species_of(c, h);
   if (s.dist == PAMTRA_B200_DIST_DISABLED) { done(0, 0); return; }
   const size_t lz = (size_t)c * Lm + z;
@@ -876,7 +876,7 @@ __global__ void k_fullspec(Batch b, Work w, pamtra_b200_settings st) {
   const int c = s_idx / ((size_t)H * Lm);
   w.slot_st[s_idx] = 0;
   w.slot_nb[s_idx] = 0;
-  if (z >= b.nlyrs[c]) return;
+  if (z >= b.layers(c)) return;
   const int nb = b.fs_nbin;
   const double* n = b.fs_n + s_idx * nb;
   double nsum = 0.0;
@@ -914,7 +914,7 @@ constexpr int COMPACT_WARPS = 32;
 // Presence of layers z0 + lane of column c (whole warp).
 __device__ __forceinline__ bool layer_present(const Batch& b, const Work& w, int c, int z, bool& fatal) {
   bool pres = false;
-  if (z < min(b.nlyrs[c], b.max_nlyrs)) {
+  if (z < b.layers(c)) {
     const int8_t* st = w.slot_st + ((size_t)c * b.max_nlyrs + z) * b.nhydro;
     for (int h = 0; h < b.nhydro; h++) {
       pres |= st[h] >= 1;

@@ -26,6 +26,12 @@ struct Batch {
   int fs_nbin;
   const double *fs_d, *fs_d_bound, *fs_n, *fs_rho, *fs_mass;
 
+  // layers of column c; 0 when k_atmo refuses its count, so that no other kernel
+  // reads or writes rows of the column (a larger count runs into its neighbour's)
+  __device__ __forceinline__ int layers(int c) const {
+    const int L = nlyrs[c];
+    return L >= 2 && L <= max_nlyrs ? L : 0;
+  }
   __device__ __forceinline__ int col_nfreq(int c) const { return nfreq ? nfreq[c] : max_nfreq; }
   __device__ __forceinline__ double freq(int c, int f) const {
     return freq_per_col ? freqs[(size_t)c * max_nfreq + f] : freqs[f];
