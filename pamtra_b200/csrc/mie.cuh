@@ -272,13 +272,15 @@ __device__ cplx eps_mix_m(cplx eps1, double mix_de) {
 
 // INT(x + 4 x**0.3334 + 2) of mie_spheres.f90.  The power in single precision
 // is good to 1e-4 here (x**0.3334 below 6); only where that could change the whole number
-// (one value in a thousand) does the double-precision one decide.
+// (one value in a thousand) does the double-precision one decide.  -1 for a size
+// parameter without a series (negative, NaN), NT_MAX or more for one too large.
 __device__ __forceinline__ int mie_nstop(double x) {
   const float xf = (float)x;
   if (xf > 1e-30f && xf < 200.0f) {
     const float v = xf + 4.0f * exp2f(0.3334f * log2f(xf)) + 2.0f, fr = v - floorf(v);
     if (fr > 1e-3f && fr < 1.0f - 1e-3f) return (int)v;
   }
+  if (!(x >= 0.0)) return -1;
   return (int)(x + 4.0 * pow(x, F(0.3334f)) + 2);
 }
 
@@ -612,9 +614,13 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
               const cplx ms = (sp_liq_ice == -1 && rho != 917.0) ? eps_mix_m(m_ice, rho) : m_ice;
               const double x = PI * dia / wl;
               int nmie = mie_nstop(x);
-              if (nmie >= NT_MAX) { nmie = NT_MAX - 1; status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE; }
-              double qe, qs, qb;
-              miecalc_slab(nmie, x, ms, col, ldc, qe, qs, qb);
+              if (nmie < 0 || nmie >= NT_MAX) {
+                nmie = nmie < 0 ? 0 : NT_MAX - 1;
+                status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;
+              }
+              // a bin without a series: no terms, no cross sections, no weight
+              double qe = 0.0, qs = 0.0, qb = 0.0;
+              if (nmie > 0) miecalc_slab(nmie, x, ms, col, ldc, qe, qs, qb);
               const double r2 = (dia / 2.0) * (dia / 2.0);
               qe = qe * r2 * PI;
               qs = qs * r2 * PI;
@@ -627,7 +633,7 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
               sqb = sqb + qb * deld;
               qb_bin = qb;
               nm = min(nmie, nterms);
-              wgt = ndens;
+              wgt = nm > 0 ? ndens : 0.0;
             }
             // per-particle cross section as back_spec / num_density of
             // src/scatProperties.f90:916 (0 / 0 = NaN for an empty bin)
