@@ -606,11 +606,7 @@ __global__ void __launch_bounds__(SymTeam<2 * N>::T) k_adding_finish(Batch b, Wo
   A::init(S, w);
   for (int unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
     const int c = unit / Fm, fi = unit % Fm;
-    if (fi >= b.col_nfreq(c) || b.col_nummu(c) != N) continue;
-    if (b.layers(c) == 0) {
-      A::put_emissivity(b, st, out, c, fi);
-      continue;
-    }
+    if (b.layers(c) == 0 || fi >= b.col_nfreq(c) || b.col_nummu(c) != N) continue;
     const float* stk = w.add_stk + (size_t)unit * STK_FLOATS;
     const int sstate = reinterpret_cast<const int*>(stk + STK_HDR)[0];
     const int status = reinterpret_cast<const int*>(stk + STK_HDR)[1];

@@ -629,17 +629,10 @@ struct Adder {
         tbo[dn_i + 1] = rad_to_tb(d1, wl);
       }
     }
-    put_emissivity(b, st, out, c, fi);
+    if (out.emissivity)
+      for (int k = t; k < 2 * N; k += T)
+        out.emissivity[(((size_t)c * 2 + k / N) * Fm + fi) * b.max_nummu + k % N] = e;
     if (t == 0 && status) atomicOr(&w.status[(size_t)c * Fm + fi], status);
-  }
-
-  // The emissivity output of a unit.  Also that of a column whose number of layers is
-  // refused: no radiance is computed for it (tb stays -9999, the status says so).
-  __device__ static __forceinline__ void put_emissivity(const Batch& b, const pamtra_b200_settings& st,
-                                                        const pamtra_b200_outputs& out, int c, int fi) {
-    if (!out.emissivity) return;
-    for (int k = threadIdx.x; k < 2 * N; k += T)
-      out.emissivity[(((size_t)c * 2 + k / N) * b.max_nfreq + fi) * b.max_nummu + k % N] = st.emissivity;
   }
 
   // quadrature nodes and the scaling of the stack's rows (1 when not SYM)
@@ -673,12 +666,8 @@ __global__ void __launch_bounds__(SymTeam<2 * N>::T, (N == 32 ? 1 : 4)) k_adding
     const int item = S.unit;
     if (item >= nitems) break;
     const int unit = item / maxseg, seg = item % maxseg, c = unit / Fm, fi = unit % Fm;
-    if (fi >= b.col_nfreq(c) || b.col_nummu(c) != N) continue;
     const int L = b.layers(c);
-    if (L == 0) {
-      if (seg == 0) A::put_emissivity(b, st, out, c, fi);
-      continue;
-    }
+    if (L == 0 || fi >= b.col_nfreq(c) || b.col_nummu(c) != N) continue;
     const int* pres = w.pres_idx + (size_t)c * Lm;
     // scattering layers of the unit, and of this segment: top-down layers k0 .. k1 - 1
     int M = 0;

@@ -934,7 +934,7 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
       launches++;
     }
   }
-  k_atmo<<<(unsigned)((C + 3) / 4), 128, 0, stream>>>(b, w); launches++;
+  k_atmo<<<(unsigned)((C + 3) / 4), 128, 0, stream>>>(b, w, st->emissivity, out->emissivity); launches++;
   const size_t ngas = C * Fm * Lm;
   launch_gas(b, w, st->lgas_extinction, st->gas_mod, ngas, stream); launches++;
   mark(ctx, stream, STG_PREP);
@@ -1546,7 +1546,7 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   const int maxseg = add_max_segments((int)Lm);
   const size_t ntb = (size_t)cc.noutlevels * 2 * cc.max_nummu * Fm * 2;
   k_fill_d<<<(unsigned)((ntb + 255) / 256), 256, 0, stream>>>(out->tb, -9999.0, ntb);
-  k_atmo<<<1, 128, 0, stream>>>(b, w);
+  k_atmo<<<1, 128, 0, stream>>>(b, w, st->emissivity, out->emissivity);
   launch_gas(b, w, st->lgas_extinction, st->gas_mod, Fm * Lm, stream);
   if (nh > 0) k_psd<<<(unsigned)((Lm * nh + PSD_WARPS - 1) / PSD_WARPS), 32 * PSD_WARPS, 0, stream>>>(b, w, *st);
   launch_compact(b, w, stream);

@@ -22,7 +22,9 @@ __device__ double e_sat_gg_water(double T) {
 // chain of logs, powers and divisions of its own, so a thread per column ran
 // 50-150 such chains one after another whatever the batch size (136 us for
 // one column of 50 layers, 750 us for 64 columns of 150; now 14 and 31 us).
-__global__ void __launch_bounds__(128) k_atmo(Batch b, Work w) {
+// A column whose layer count is refused ends here: its emissivity output, which the
+// end of the adding writes for the others, is written here.
+__global__ void __launch_bounds__(128) k_atmo(Batch b, Work w, double emissivity, double* out_emissivity) {
   const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (c >= b.ncol) return;
   const int Lm = b.max_nlyrs, L = b.nlyrs[c];
@@ -50,6 +52,11 @@ __global__ void __launch_bounds__(128) k_atmo(Batch b, Work w) {
     if (lane == 0) w.col_status[c] |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;
     const int nf = min(b.col_nfreq(c), b.max_nfreq);
     for (int f = lane; f < nf; f += 32) w.status[(size_t)c * b.max_nfreq + f] |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;
+    if (bad_l && out_emissivity && (nbit & b.nummu_mask))
+      for (int e = lane; e < 2 * nf * nm; e += 32) {
+        const int j = e % nm, f = (e / nm) % nf, q = e / (nm * nf);
+        out_emissivity[(((size_t)c * 2 + q) * b.max_nfreq + f) * b.max_nummu + j] = emissivity;
+      }
     if (bad_l) return;
   }
   // layer heights first (only needs levels), then the level variables
