@@ -609,18 +609,20 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
             deld = bdd[ir];
             double rho = brho[ir], dia = bd[ir];
             ndens = bnd[ir] / deld;
+            int nmie = -1;
+            double x = 0.0;
             if (ndens > 0) {
               dens_diam(ir, rho, dia);
+              x = PI * dia / wl;
+              nmie = mie_nstop(x);
+              // a bin without a series takes no part, one of a longer series than the tables hold ends there
+              if (nmie < 0 || nmie >= NT_MAX) status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;
+            }
+            if (nmie >= 0) {
+              nmie = min(nmie, NT_MAX - 1);
               const cplx ms = (sp_liq_ice == -1 && rho != 917.0) ? eps_mix_m(m_ice, rho) : m_ice;
-              const double x = PI * dia / wl;
-              int nmie = mie_nstop(x);
-              if (nmie < 0 || nmie >= NT_MAX) {
-                nmie = nmie < 0 ? 0 : NT_MAX - 1;
-                status |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;
-              }
-              // a bin without a series: no terms, no cross sections, no weight
-              double qe = 0.0, qs = 0.0, qb = 0.0;
-              if (nmie > 0) miecalc_slab(nmie, x, ms, col, ldc, qe, qs, qb);
+              double qe, qs, qb;
+              miecalc_slab(nmie, x, ms, col, ldc, qe, qs, qb);
               const double r2 = (dia / 2.0) * (dia / 2.0);
               qe = qe * r2 * PI;
               qs = qs * r2 * PI;
@@ -633,7 +635,7 @@ __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_sett
               sqb = sqb + qb * deld;
               qb_bin = qb;
               nm = min(nmie, nterms);
-              wgt = nm > 0 ? ndens : 0.0;
+              wgt = ndens;
             }
             // per-particle cross section as back_spec / num_density of
             // src/scatProperties.f90:916 (0 / 0 = NaN for an empty bin)
