@@ -154,11 +154,12 @@ __global__ void __launch_bounds__(128) k_scat_weights(double* __restrict__ tab, 
 }
 
 // Mark the numpts tables of N filled by k_scat_weights (run by one block of
-// the kernel that follows it on the stream).
+// the kernel that follows it on the stream).  Without a table (its allocation
+// failed) nothing was filled: a later call that gets one fills it.
 template <int N>
 __device__ __forceinline__ void scat_weights_mark_ready(const Work& w) {
   const int ni = nmu_index(N);
-  if (blockIdx.x == 0 && w.wt_need)
+  if (blockIdx.x == 0 && w.wt_need && w.wtab[ni])
     for (int i = threadIdx.x; i < SCAT_NPI; i += blockDim.x)
       if (w.wt_need[ni * SCAT_NPI + i]) w.wt_ready[ni * SCAT_NPI + i] = 1;
 }
