@@ -178,6 +178,7 @@ struct TmShared {
   double accs[8], qe[3], qs[3];
   double piv[2];
   int ok[3], len[3][2];
+  int sing[3];  // a pivot of the step vanished
   int pivrow;
   int particle;
   long long rec;
@@ -657,6 +658,7 @@ __device__ void tm_steps(const TmStep (&st)[NC], const TmPart& A, TmShared& sh, 
       const bool ok = tm_lengths(ta, st[c].nx, A, l1, l2);
       if (lane == 0) {
         sh.ok[c] = ok;
+        sh.sing[c] = 0;
         sh.len[c][0] = l1;
         sh.len[c][1] = l2;
       }
@@ -692,6 +694,8 @@ __device__ void tm_steps(const TmStep (&st)[NC], const TmPart& A, TmShared& sh, 
     first += np;
   }
   __syncthreads();
+  // sh.ok stays as it is until all warps are through: a lane that read it later
+  // than its neighbours would miss the shuffles they wait in
   for (int k = warp; k < 4 * NC; k += NW) {
     const int c = k >> 2;
     if (!sh.ok[c]) continue;
@@ -700,13 +704,16 @@ __device__ void tm_steps(const TmStep (&st)[NC], const TmPart& A, TmShared& sh, 
       if (j == c) {
         const TmSystems sy(0, st[j].nx);
         const int q = sy.size(k & 3);
-        if (q > 0 && !tm_eliminate<1>(tm_aug(st[j].s) + sy.base(k & 3), q, sh) && lane == 0) sh.ok[c] = 0;
+        if (q > 0 && !tm_eliminate<1>(tm_aug(st[j].s) + sy.base(k & 3), q, sh) && lane == 0) sh.sing[c] = 1;
       }
   }
   __syncthreads();
 #pragma unroll
   for (int c = 0; c < NC; c++)
-    if (t == 32 * (c % NW) && sh.ok[c]) tm_sums(tm_aug(st[c].s), st[c].nx, sh.qe[c], sh.qs[c]);
+    if (t == 32 * (c % NW) && sh.ok[c]) {
+      if (sh.sing[c]) sh.ok[c] = 0;
+      else tm_sums(tm_aug(st[c].s), st[c].nx, sh.qe[c], sh.qs[c]);
+    }
   __syncthreads();
 }
 

@@ -68,3 +68,22 @@ def test_gpu_tmatrix_record_rounds(oracle_mod):
         for c in (0, 1):
             sel = good & (np.arange(n) % 2 == c)
             assert np.all(v[sel] == v[c]), (k, c)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("d", [1e-80, 1e-120])
+def test_gpu_tmatrix_vanishing_pivots(oracle_mod, d):
+    """Particles so small that the Bessel functions overflow: every system of all
+    steps of the side-by-side search loses its pivots at once.  The bins say
+    FATAL | ST_RANGE, and the bins beside them keep their bytes."""
+    fine = _ice((0.3, 2.0), 0.8, 0.0)
+    mixed = {k: (v[:1] + [w] * 4 + v[1:] if isinstance(v, list) else v)
+             for k, v, w in ((k, fine[k], fine[k][0] if isinstance(fine[k], list) else None) for k in fine)}
+    mixed["dmax"][1:5] = [d] * 4
+    want = _run_gpu([fine], 3, 8)
+    out = _run_gpu([mixed], 7, 8)
+    assert int(out["status"][0]) == (2 | 0x10000)
+    assert np.all(out["nmax"][0, 1:5] < 0)
+    for k in ("scatter_matrix", "extinct_matrix", "emis_vector", "sback"):
+        assert np.array_equal(out[k][0], want[k][0]), k
+    assert np.array_equal(np.delete(out["back_spec"][0], range(1, 5)), want["back_spec"][0])
