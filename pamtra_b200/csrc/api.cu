@@ -170,7 +170,8 @@ __global__ void k_ssp_out(Batch b, Work w, pamtra_b200_outputs out) {
   const int Lm = b.max_nlyrs, Fm = b.max_nfreq;
   if (idx >= (size_t)b.ncol * Fm * Lm) return;
   const int z = idx % Lm, f = (idx / Lm) % Fm, c = idx / ((size_t)Lm * Fm);
-  const int p = (z < b.layers(c)) ? w.pres_idx[(size_t)c * Lm + z] : -1;
+  // no item was computed past the column's frequencies
+  const int p = (z < b.layers(c) && f < b.col_nfreq(c)) ? w.pres_idx[(size_t)c * Lm + z] : -1;
   const size_t item = (size_t)p * Fm + f;
   if (out.kexttot) out.kexttot[idx] = (p >= 0) ? w.m_kext[item] : 0.0;
   if (out.salbedo) out.salbedo[idx] = (p >= 0) ? w.m_salb[item] : 0.0;

@@ -56,3 +56,22 @@ def test_refused_columns_leave_the_others_alone(native, nummu, refused):
                 assert np.array_equal(got["tb"][c], good["tb"][c]), (prec, c)
                 for k in ("status", "kextatmo", "kexttot", "salbedo", "num_doubles", "ze", "att_hydro", "att_atmo"):
                     assert np.array_equal(got[k][c, :nf], good[k][c, :nf], equal_nan=True), (prec, k, c)
+
+
+def test_outputs_past_a_columns_frequencies(native):
+    """Columns of fewer frequencies than the batch's widest: the per-layer outputs
+    past them say that there is no layer (0, 0, -1), whatever the scratch held."""
+    import torch
+    dev = torch.device("cuda", 0)
+    eng = native.Engine(0)
+    for seed, nfr in ((70, (6, 6)), (71, (1, 6))):  # the first batch leaves its items in the scratch
+        b = wl.uneven_batch(6, seed=seed, nummu_choices=(8,), nfreq_range=nfr)
+        out = b.alloc_outputs(dev, ssp=True)
+        pbatch.run(b, 0, out, eng=eng)
+        torch.cuda.synchronize()
+    out = {k: v.cpu().numpy() for k, v in out.items()}
+    eng.close()
+    past = np.arange(out["status"].shape[1])[None, :] >= b.host["nfreq"][:, None]
+    assert past.any() and (out["num_doubles"][~past] >= 0).any()
+    for k, v in (("kexttot", 0.0), ("salbedo", 0.0), ("num_doubles", -1)):
+        assert np.all(out[k][past] == v), k
