@@ -915,7 +915,7 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   for (int i = 0; i < 3; i++) w.wtab[i] = ctx->wt_flags ? ctx->wtab[i] : nullptr;
   w.wt_need = ctx->wt_flags;
   w.wt_ready = ctx->wt_flags ? ctx->wt_flags + 3 * SCAT_NPI : nullptr;
-  w.gq_x = ctx->gq_x; w.gq_w = ctx->gq_w; w.gq_max = GQ_MAX; w.mie_tab = ctx->mie_tab; w.lob_mu = ctx->lob_mu; w.lob_w = ctx->lob_w;
+  w.gq_w = ctx->gq_w; w.gq_max = GQ_MAX; w.mie_tab = ctx->mie_tab; w.lob_mu = ctx->lob_mu; w.lob_w = ctx->lob_w;
 
   int launches = 0;
   ctx->nev = 0;
@@ -1536,7 +1536,7 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   w.seg_cnt = (int*)(A + pl.o_segcnt);
   w.spin_limit = tc::MBAR_SPIN_LIMIT;
   w.mie_slab = (double*)(A + pl.o_mieslab); w.mie_nslab = pl.mie_nslab;
-  w.gq_x = D.tables; w.gq_w = D.tables + gqn; w.gq_max = NOALLOC_GQ; w.mie_tab = D.mie_tab;
+  w.gq_w = D.tables + gqn; w.gq_max = NOALLOC_GQ; w.mie_tab = D.mie_tab;
   w.lob_mu = D.tables + 2 * gqn; w.lob_w = D.tables + 2 * gqn + 56;
   const size_t Lm = cc.max_nlyrs, Fm = cc.max_nfreq;
   // the scratch keeps the previous call's contents: clear what must start at zero

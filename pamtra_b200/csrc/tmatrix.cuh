@@ -175,7 +175,7 @@ struct TmArgs {
 __device__ __forceinline__ int tm_inm1(double xev) { return max(4, (int)(xev + 4.05 * pow(xev, 0.333333))); }
 
 struct TmShared {
-  double accs[8], qe[3], qs[3];
+  double qe[3], qs[3];
   double piv[2];
   int ok[3], len[3][2];
   int sing[3];  // a pivot of the step vanished

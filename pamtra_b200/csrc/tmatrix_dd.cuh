@@ -25,6 +25,7 @@ namespace pb {
 // Whole CTA; false when the reference would stop.
 __device__ bool tdd_setup(double* sd, TmShared& sh, int nmax, int ngauss, double lam, double mrr, double mri,
                           double rev, double eps) {
+  __shared__ double size[TM_THREADS / 32];
   const int t = threadIdx.x, ng = 2 * ngauss;
   if (t < (ng + 1) / 2) tdd_gauss_pair(sd, ng, t);
   __syncthreads();
@@ -32,10 +33,10 @@ __device__ bool tdd_setup(double* sd, TmShared& sh, int nmax, int ngauss, double
   __syncthreads();
   double ta = (t < ng) ? tdd_size_node(sd, t, lam, mrr, mri) : 0.0;
   for (int o = 16; o > 0; o >>= 1) ta = fmax(ta, __shfl_xor_sync(0xffffffffu, ta, o));
-  if ((t & 31) == 0) sh.accs[t >> 5] = ta;
+  if ((t & 31) == 0) size[t >> 5] = ta;
   __syncthreads();
   ta = 0.0;
-  for (int w = 0; w < TM_THREADS / 32; w++) ta = fmax(ta, sh.accs[w]);
+  for (int w = 0; w < TM_THREADS / 32; w++) ta = fmax(ta, size[w]);
   int nnmax1 = 0, nnmax2 = 0;
   const bool ok = tdd_lengths(ta, nmax, mrr, mri, &nnmax1, &nnmax2);
   __syncthreads();

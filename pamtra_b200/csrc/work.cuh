@@ -94,8 +94,7 @@ struct Work {
   int* status;                         // [C][Fm]
   int* col_status;                     // [C]
   // quadrature tables
-  const double* gq_x;                  // Gauss-Legendre nodes, packed: nquad=q at offset q*(q-1)/2
-  const double* gq_w;
+  const double* gq_w;                  // Gauss-Legendre weights, packed: nquad=q at offset q*(q-1)/2
   int gq_max;
   const double* mie_tab;               // angular tables of k_mie (MIE_TAB doubles)
   const double* lob_mu;                // Lobatto nodes for N = 8,16,32 at offsets 0, 8, 24
