@@ -195,9 +195,9 @@ __device__ __forceinline__ void mm_unit(const double* A, const double* B, double
       }
 }
 
-// (I - P)^-1 of one unit by its two warps, the Neumann series of
-// inv_iminus() (same plan from the infinity norm, Horner or repeated
-// squaring, same products): returns the buffer holding the inverse (P or
+// (I - P)^-1 of one unit by its two warps: a Neumann series whose length
+// follows from the infinity norm (remainder below 2^-54), by Horner or repeated
+// squaring, whichever takes fewer products: returns the buffer holding the inverse (P or
 // G), or nullptr when the norm asks for Gauss-Jordan (P left untouched).
 __device__ __forceinline__ double* inv_unit(double* P, double* G, int wl, int mi) {
   constexpr int LD = Team<32>::LD;
@@ -520,8 +520,8 @@ __global__ void __launch_bounds__(128, 2) k_adding_tc(Batch b, Work w, pamtra_b2
           }
           if (u == 0) s_gj[mi] = gj;
           __syncthreads();
-          // ||Gin|| >= 0.74: Gauss-Jordan with partial pivoting, one unit at a
-          // time with the whole CTA (the fallback of inv_iminus)
+          // ||Gin|| above about 0.56: Gauss-Jordan with partial pivoting, one unit at a
+          // time with the whole CTA
           for (int i = 0; i < 2; i++) {
             if (!s_gj[i]) continue;
             AddTcInv& F = Q.u.fp[i];

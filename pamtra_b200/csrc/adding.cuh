@@ -15,11 +15,14 @@
 // split-precision doubling, symmetric to FP32 rounding only): unscaled and in full.
 //
 // Layout and roles are those of SymTeam: n / 8 warps, warp i owns the strip of
-// rows 8i .. 8i + 7 of every result and every product chain stays in its
-// registers; R- (and T-) are read by their owner alone and live in registers
-// for the whole unit.  Shared memory holds R+, T+, the layer's R and T and
-// two work matrices (R1p R2m and its powers): 49 KB for n = 32, four CTAs per
-// SM (two with ten matrices); n = 64 fits without the global scratch it took.
+// rows 8i .. 8i + 7 of every result; the strip of a product is the left factor
+// of the next without an exchange, and R- (and T-), which their owner alone reads,
+// have no place in shared memory.  That holds the registers full: 128 at four CTAs per
+// SM for n = 32, 255 for n = 64, and the rest spills to local memory (bytes of
+// stores / loads per thread: <16, true> 406 / 452, <16, false> 634 / 612, <32, true>
+// 950 / 992, <32, false> 2498 / 2556; NUMMU 8 none).  Shared memory holds R+, T+,
+// the layer's R and T and two work matrices (R1p R2m and its powers): 49 KB
+// for n = 32; n = 64 fits without the global scratch it took.
 //
 // A unit's layers go in segments of about sqrt(M) of its M scattering layers
 // (adding is associative), each a work item of its own; the CTA that finishes
@@ -27,7 +30,8 @@
 // the same, and a column's chain of M dependent combines becomes one of about
 // 2 sqrt(M).  Segments follow from the column alone, so results do not
 // depend on the batch.  What bounds it: the chain of dependent products of a
-// combine at 16 warps per SM.  Adding stage, before (one chain per unit,
+// combine at 16 warps per SM (8 for n = 64): FP64 tensor pipe 48 %, 65 % for n = 64, with
+// the barriers and spills between.  Adding stage, before (one chain per unit,
 // twelve or ten full products, two CTAs per SM) and now: one column 0.43 ->
 // 0.16 ms, 1500 columns x 50 layers x 4 frequencies 6.4 -> 4.4 ms (three
 // CTAs per SM 4.6), 64 columns of 150 layers 1.65 -> 1.02 ms, 40 columns of
@@ -39,8 +43,9 @@
 
 namespace pb {
 
-// Segments of a unit with M scattering layers: lengths of at least four, so
-// a segment's stack fits the first two of its layer records.
+// Segments of a unit with M scattering layers, of about max(4, sqrt(M)) layers each
+// and at least three (M = 9: 3, 3, 3); a segment's stack needs the first two of its
+// layer records.
 __host__ __device__ __forceinline__ int add_segments(int M) {
   if (M < 8) return 1;
   int len = 4;

@@ -360,7 +360,9 @@ __device__ __noinline__ void miecalc_slab(int nterms, double x, cplx mn, double*
     next += ldc;
     if (n < nterms) dv = *reinterpret_cast<const double2*>(next);  // travels during this term
     // a_n and b_n: numerators over denominators z as (numerator conj(z)) / |z|^2, both by one
-    // reciprocal (|z| stays within a few hundred orders of magnitude of 1)
+    // reciprocal.  |za|^2 |zb|^2 would overflow from |z| of about 1e77: xi is held in REAL(4)
+    // range (below 3.4e38, else infinite as in the reference), which a size parameter of 1e-19
+    // reaches at n = 2, where |z| is 1e58.
     const double nx = rn * xinv;
     const cplx ca = cmk(fma(dn.re, minv.re, fma(-dn.im, minv.im, nx)), fma(dn.re, minv.im, dn.im * minv.re));
     const cplx cb = cmk(fma(m.re, dn.re, fma(-m.im, dn.im, nx)), fma(m.re, dn.im, m.im * dn.re));
@@ -494,13 +496,16 @@ __device__ __noinline__ void mie_pass_sums(MieSmem& S, const double* __restrict_
 // phase-function sums of the pass are formed on the FP64 tensor cores (phase B,
 // mie_pass_sums).  The Legendre projection runs lanes over orders, the
 // quadrature points folded about 0 (P_l is even or odd) and P_l from a table.
-// The species sums accumulate in the item's coefficient output row.
+// The species sums accumulate behind the coefficients in the warp's slab and go to the
+// item's coefficient row at the end.
 // Bound by the FP64 pipes, which the scalar series of phase A and the DMMAs of
-// phase B share, and by the latency of both at 16 warps per SM (128 registers):
+// phase B share, and by the latency of both at 16 warps per SM (128 registers, with
+// 296 bytes of spill stores and 364 of loads per thread):
 // Mie stage at 1500 columns of 6-term species 6.8 ms with FP64 FMAs per (four
 // bins, angle) and warp sums per Legendre order, now 4.9 ms; 40 columns of
 // 20-term species with 200 bins 6.2 ms, now 3.6 ms.
-// One tile pair (NP = 1); two spill (8.2 and 6.0 ms before the series were trimmed).
+// One tile pair (NP = 1); two spill more (352 and 476 bytes; 8.2 and 6.0 ms against 6.4 and
+// 4.3 before the series were trimmed).
 template <int NP>
 __global__ void __maxnreg__(MIE_MAXNREG) k_mie(Batch b, Work w, pamtra_b200_settings st) {
   extern __shared__ double smem_raw[];

@@ -176,10 +176,10 @@ struct LayerItem {
 // shared memory.  Returns false when the item is not for this N.
 // Latency of one CTA, while its neighbours double: the table rows of several
 // orders travel at once, the Planck functions run in the last warp beside the
-// coefficients, norms eight lanes to a row. 
-// Set-up of an item of 1500 columns (N = 16) 46 k -> 23 k cycles, of a Mie-heavy one
-// 62 k -> 29 k; layer stage 22.0 -> 21.8 ms, mixed NUMMU 19.7 -> 19.4 (split
-// form 14.2 -> 13.7), split form 13.0 -> 12.85: the doubling of the others takes up the rest.
+// coefficients, norms eight lanes to a row.
+// Layer stage, 1500 columns (N = 16) 22.0 -> 21.8 ms, mixed NUMMU 19.7 -> 19.4 (split
+// form 14.2 -> 13.7), split form 13.0 -> 12.85: the set-up halved, but the doubling of the
+// CTAs beside it takes up most of that.
 template <int N, class SM, int T = RTCfg<N>::T>
 __device__ __forceinline__ bool layer_setup(const Batch& b, const Work& w, const pamtra_b200_settings& st,
                                             double* __restrict__ ssp_scat, SM& S, int item,
@@ -677,7 +677,8 @@ __global__ void __launch_bounds__(LayerCfg<N>::T, LayerCfg<N>::CTAS) k_layer(Bat
           for (int k = 1; k < (n + 31) / 32; k++) rs = fmax(rs, S.inv.cand_v[k]);
           nrm = fmin(nrm, rs);
         }
-        // further terms: kh by Horner (remainder nrm^(kh + 2)) or m - 1 squarings (remainder nrm^(2^m))
+        // further terms: kh by Horner (remainder nrm^(kh + 2) below 5e-17) or m - 1 squarings
+        // (remainder nrm^(2^m), m the first with nrm^(2^(m-1)) below 5e-17: one factor to spare)
         for (double pw = nrm; pw > 5.0e-17 && m < 8; m++) pw = pw * pw;
         for (double ph = nrm * nrm; ph > 5.0e-17 && kh < 2 * (m - 1); kh++) ph = ph * nrm;
       }
@@ -716,7 +717,7 @@ __global__ void __launch_bounds__(LayerCfg<N>::T, LayerCfg<N>::CTAS) k_layer(Bat
         for (int k = 0; k < kh; k++) term(true);
         tiles += (kh + 1) * NB * NB;
       } else {
-        // W = T (I + X)(I + X^2)(I + X^4)...
+        // W = T (I + X)(I + X^2)(I + X^4)..., m factors (the remainder would allow m - 1)
         term(false);
         for (int k = 1; k < m; k++) {
           double x[D + 1][2];

@@ -35,8 +35,9 @@
 // 1024 upright particles of NMAX 5 - 14 (1.2 - 6 mm, 89 GHz): 8.6 ms with one
 // barrier chain per particle and AMPL per pair, now 0.88 ms; 96 canted ones 39 ms,
 // now 0.43 ms (0.99 and 0.59 ms with all 30 azimuths).  Bound by latency (pivots,
-// recurrences and phases that follow one another: FP64 pipe 24 % while a CTA is
-// busy).  With 30 azimuths, four warps per CTA and four CTAs per SM: 1.16 and
+// recurrences and phases that follow one another: FP64 pipe 19 % of the solve's active
+// cycles, the largest stall at the CTA's barriers; 30 % of the amplitudes', which wait for
+// loads).  With 30 azimuths, four warps per CTA and four CTAs per SM: 1.16 and
 // 0.74 ms; one order after another with a warp per solve: 1.36 and 0.72 ms.
 // The reference computes the solve in REAL*16; FP64 here agrees with it to
 // about 1e-12 relative on microwave hydrometeors, below the single-precision
@@ -1441,9 +1442,8 @@ __device__ void tm_particle(const TmArgs& A, double* s, const TmSlot& L, TmShare
   }
 }
 
-// Persistent CTAs over the particles of a round, one scratch slot
-// each.  Eight warps when there are at most two particles per SM (the m >= 1
-// solves of one run side by side), four otherwise (more particles in flight).
+// Persistent CTAs of eight warps over the particles of a round, one scratch slot
+// each.
 __global__ void __launch_bounds__(TM_THREADS, 2) k_tmatrix(TmArgs A) {
   __shared__ TmShared sh;
   const TmSlot L = tm_slot(A.nummu);
