@@ -302,8 +302,9 @@ def fp64_peak_tflops(dev):
 
 
 # k_layer<16> DRAM traffic per (layer, frequency) item: ncu capture of the
-# 256-column run (21,504 items): 17.7 MB read + 348.3 MB written per launch
-LAYER_TRAFFIC_PER_ITEM = (17.698560e6 + 348.297472e6) / 21504
+# 256-column run (21,504 items): 13.7 MB read + 308.1 MB written per launch
+# (profiles/k_layer_fp64_dmma.md)
+LAYER_TRAFFIC_PER_ITEM = (13.749504e6 + 308.110848e6) / 21504
 
 
 def layer_flops(nd, N):
@@ -402,7 +403,8 @@ def _target_shape(args, local, eng, stream):
             "tb_err_3xtf32_vs_fp64_K": split_err, "stage_ms_3xtf32": sstages,
             "unit": "solves/s", "batched_ms_per_step": float(np.mean(ms)), "status_nonzero": st_bad,
             "plain_sample_columns": 16, "plain_vs_batched_fp64_tb_max_diff_K": plain_diff,
-            "forms": "batched FP64 (PREC_FP64_BATCHED); plain: one column per call (PREC_FP64, the same kernels)"}
+            "forms": "batched FP64 (PREC_FP64_BATCHED); plain: one column per call (PREC_FP64, the same kernels: "
+                     "plain_vs_batched_fp64_tb_max_diff_K checks batch independence)"}
 
 
 def _config_line(name, b, local, eng, stream, pool, nplain=8, reps=1, noracle=8):
@@ -808,7 +810,8 @@ def main():
         e.record(stream)
     e.synchronize()
     plain_value = nplain * len(FREQS) / (s.elapsed_time(e) * 1e-3)
-    # the plain form on the first columns of the batch: agreement with the batched form
+    # the plain form on the first columns of the batch: the same kernels, so that a
+    # difference would mean that a column depends on the batch it is in
     tb_b = out["tb"].cpu().numpy()
     plain_diff = 0.0
     for c in range(4):
@@ -840,23 +843,24 @@ def main():
     peak = fp64_peak_tflops(dev)
     t_layer = stage_tot.get("layer", 0.0) / args.steps * 1e-3
     flops = layer_flops(nd, 16)
-    achieved = flops / t_layer / 1e12 if t_layer > 0 else 0.0
+    algorithmic = flops / t_layer / 1e12 if t_layer > 0 else 0.0
+    executed = 2.0 * 32 ** 3 * layer_products / t_layer / 1e12 if t_layer > 0 else 0.0
     items = int(np.count_nonzero(nd >= 0))
     roofline = {"bound": "tensor", "pipe": "FP64 tensor (DMMA)", "kernel": "k_layer<16> (scatcnv + init + doubling)",
-                "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
+                "achieved": executed, "peak": peak, "unit": "TFLOP/s", "frac": executed / peak if peak else None,
                 "traffic": LAYER_TRAFFIC_PER_ITEM * items,
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum of one launch at 256 columns "
                                   "(21,504 items), scaled by the %d items of this launch" % items,
                 "peak_source": "cuBLAS DGEMM 8192^3 measured in this run (FP64 tensor pipe); "
                                "MEASURED_PEAKS.json carries bf16 and HBM only",
-                "flops_per_launch": flops, "kernel_ms": t_layer * 1e3,
-                "achieved_executed": 2.0 * 32 ** 3 * layer_products / t_layer / 1e12 if t_layer > 0 else None,
-                "executed_products_per_launch": layer_products,
-                "executed_note": "n x n products the kernel issued (a symmetric one counts its computed tiles; the "
-                                 "series with them, Gauss-Jordan as one), 2 n^3 FLOP each, n = 32; the algorithmic "
-                                 "figure counts 6 products and one inverse per doubling"}
-    roofline["frac_executed"] = roofline["achieved_executed"] / peak if peak and roofline["achieved_executed"] \
-        else None
+                "kernel_ms": t_layer * 1e3, "products_per_launch": layer_products,
+                "flops_per_launch": 2.0 * 32 ** 3 * layer_products,
+                "achieved_note": "n x n products the kernel issued (a symmetric one counts its computed tiles; the "
+                                 "series with them, Gauss-Jordan as one), 2 n^3 FLOP each, n = 32",
+                "algorithmic": {"achieved": algorithmic, "flops_per_launch": flops,
+                                "frac": algorithmic / peak if peak else None,
+                                "note": "counting 6 full products and one inverse per doubling, of which the "
+                                        "symmetric form issues about 3.9 products: not a rate of the hardware"}}
     # ---- CPU baseline + TB error vs the oracle on the same columns
     cpu = None
     tb_err = None
@@ -891,7 +895,9 @@ def main():
         "clocks": clocks,
         "plain_fp64": {"value": plain_value, "unit": "solves/s",
                        "form": "one column per call, FP64 (PREC_FP64)",
-                       "tb_max_diff_vs_batched_K": plain_diff},
+                       "tb_max_diff_vs_batched_K": plain_diff,
+                       "tb_max_diff_note": "same kernels: a column alone against the same column in the batch "
+                                           "(batch independence)"},
         "batched_form": "FP64 (PREC_FP64_BATCHED)",
         "graph_replay": {"value": graph_value, "unit": "solves/s", "ms_per_step": float(np.mean(g_ms)),
                          "tb_equals_direct": graph_same,
