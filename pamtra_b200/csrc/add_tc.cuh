@@ -299,11 +299,11 @@ __global__ void __launch_bounds__(128, 2) k_adding_tc(Batch b, Work w, pamtra_b2
     if (unit < nunits) {
       c = unit / Fm;
       fi = unit % Fm;
-      L = b.layers(c);
-      valid = L > 0 && fi < b.col_nfreq(c) && b.col_nummu(c) == N;
+      valid = fi < b.col_nfreq(c) && w.col_nmu[c] == N;
     }
     double wl = 0.0;
     if (valid) {
+      L = b.nlyrs[c];
       wl = C_LIGHT / (b.freq(c, fi) * 1.e3);
       status = w.col_status[c];
     }
@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(SymTeam<2 * N>::T) k_adding_finish(Batch b, Wo
   A::init(S, w);
   for (int unit = blockIdx.x; unit < nunits; unit += gridDim.x) {
     const int c = unit / Fm, fi = unit % Fm;
-    if (b.layers(c) == 0 || fi >= b.col_nfreq(c) || b.col_nummu(c) != N) continue;
+    if (fi >= b.col_nfreq(c) || w.col_nmu[c] != N) continue;
     const float* stk = w.add_stk + (size_t)unit * STK_FLOATS;
     const int sstate = reinterpret_cast<const int*>(stk + STK_HDR)[0];
     const int status = reinterpret_cast<const int*>(stk + STK_HDR)[1];

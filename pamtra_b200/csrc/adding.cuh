@@ -19,8 +19,8 @@
 // of the next without an exchange, and R- (and T-), which their owner alone reads,
 // have no place in shared memory.  That holds the registers full: 128 at four CTAs per
 // SM for n = 32, 255 for n = 64, and the rest spills to local memory (bytes of
-// stores / loads per thread: <16, true> 406 / 452, <16, false> 634 / 612, <32, true>
-// 950 / 992, <32, false> 2498 / 2556; NUMMU 8 none).  Shared memory holds R+, T+,
+// stores / loads per thread: <16, true> 390 / 432, <16, false> 634 / 608, <32, true>
+// 946 / 984, <32, false> 2222 / 2236; NUMMU 8 none).  Shared memory holds R+, T+,
 // the layer's R and T and two work matrices (R1p R2m and its powers): 49 KB
 // for n = 32; n = 64 fits without the global scratch it took.
 //
@@ -537,7 +537,7 @@ struct Adder {
                                                 const pamtra_b200_outputs& out, SM& S, const RG& G, int i, int c,
                                                 int fi, bool scat, int status) {
     const int t = threadIdx.x, lane = t & 31, g = lane >> 2, q = lane & 3, row = 8 * i + g;
-    const int Fm = b.max_nfreq, L = b.layers(c);
+    const int Fm = b.max_nfreq, L = b.nlyrs[c];
     const double wl = C_LIGHT / (b.freq(c, fi) * 1.e3);
     const char refl = (char)b.sfc_refl[c];
     const double e = st.emissivity, rr = 1.0 - e;
@@ -671,8 +671,8 @@ __global__ void __launch_bounds__(SymTeam<2 * N>::T, (N == 32 ? 1 : 4)) k_adding
     const int item = S.unit;
     if (item >= nitems) break;
     const int unit = item / maxseg, seg = item % maxseg, c = unit / Fm, fi = unit % Fm;
-    const int L = b.layers(c);
-    if (L == 0 || fi >= b.col_nfreq(c) || b.col_nummu(c) != N) continue;
+    if (fi >= b.col_nfreq(c) || w.col_nmu[c] != N) continue;
+    const int L = b.nlyrs[c];
     const int* pres = w.pres_idx + (size_t)c * Lm;
     // scattering layers of the unit, and of this segment: top-down layers k0 .. k1 - 1
     int M = 0;

@@ -240,7 +240,7 @@ struct Plan {
   size_t o_hgt_lev, o_temp_lev, o_temp, o_press, o_rho_vap, o_q_hum, o_vap, o_gtemp, o_outlev, o_kgas;
   size_t o_slot_st, o_slot_nb, o_bd, o_bdd, o_bnd, o_brho, o_bmass;
   size_t o_pres_idx, o_plist, o_counters, o_mkext, o_msalb, o_mback, o_mrefr, o_mnleg, o_mlegen, o_lay, o_laynd, o_status,
-      o_colst, o_colcnt;
+      o_colst, o_colcnt, o_colnmu;
   size_t o_species, o_segcnt, o_mieslab, o_addstk;
   int mie_nslab;  // k_mie warps the slabs are sized for
   bool f32_coef;
@@ -309,6 +309,7 @@ Plan make_plan(const pamtra_b200_columns* c, int default_nummu, int sms, int mie
   p.o_status = take(C * Fm * 4);
   p.o_colst = take(C * 4);
   p.o_colcnt = take(C * 4);
+  p.o_colnmu = take(C * 4);
   p.o_species = take(std::max<size_t>(nsp, 1) * sizeof(pamtra_b200_species));
   p.o_segcnt = take(C * Fm * 4);
   // one slab per k_mie warp; more warps than (layer, frequency) items would idle
@@ -894,7 +895,7 @@ int32_t pamtra_b200_run(pamtra_b200_ctx* ctx, const pamtra_b200_settings* st, co
   w.lay = (double*)(A + pl.o_lay); w.lay_stride = pl.lay_stride; w.lay_nd = (int*)(A + pl.o_laynd);
   w.lay32 = pl.tc_add ? 1 : 0;
   w.add_stk = pl.tc_add ? (float*)(A + pl.o_addstk) : nullptr;
-  w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst); w.col_cnt = (int*)(A + pl.o_colcnt);
+  w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst); w.col_cnt = (int*)(A + pl.o_colcnt); w.col_nmu = (int*)(A + pl.o_colnmu);
   w.seg_cnt = (int*)(A + pl.o_segcnt);
   w.mie_slab = (double*)(A + pl.o_mieslab); w.mie_nslab = pl.mie_nslab;
   w.spin_limit = ctx->spin_limit;
@@ -1532,7 +1533,7 @@ extern "C" int32_t pamtra_b200_run_noalloc(const pamtra_b200_settings* st, const
   w.m_legen = pl.f32_coef ? nullptr : (double*)(A + pl.o_mlegen);
   w.m_legen32 = pl.f32_coef ? (float*)(A + pl.o_mlegen) : nullptr;
   w.lay = (double*)(A + pl.o_lay); w.lay_stride = pl.lay_stride; w.lay_nd = (int*)(A + pl.o_laynd);
-  w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst); w.col_cnt = (int*)(A + pl.o_colcnt);
+  w.status = (int*)(A + pl.o_status); w.col_status = (int*)(A + pl.o_colst); w.col_cnt = (int*)(A + pl.o_colcnt); w.col_nmu = (int*)(A + pl.o_colnmu);
   w.seg_cnt = (int*)(A + pl.o_segcnt);
   w.spin_limit = tc::MBAR_SPIN_LIMIT;
   w.mie_slab = (double*)(A + pl.o_mieslab); w.mie_nslab = pl.mie_nslab;

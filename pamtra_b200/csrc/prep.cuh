@@ -48,7 +48,9 @@ __global__ void __launch_bounds__(128) k_atmo(Batch b, Work w, double emissivity
   const int nm = b.col_nummu(c);
   const int nbit = (nm == 8) ? 1 : (nm == 16) ? 2 : (nm == 32) ? 4 : 0;
   const bool bad_l = L < 2 || L > Lm;
-  if (bad_l || !(nbit & b.nummu_mask) || nm > b.max_nummu) {
+  const bool refused = bad_l || !(nbit & b.nummu_mask) || nm > b.max_nummu;
+  if (lane == 0) w.col_nmu[c] = refused ? 0 : nm;
+  if (refused) {
     if (lane == 0) w.col_status[c] |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;
     const int nf = min(b.col_nfreq(c), b.max_nfreq);
     for (int f = lane; f < nf; f += 32) w.status[(size_t)c * b.max_nfreq + f] |= PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE;

@@ -93,6 +93,7 @@ struct Work {
   // status
   int* status;                         // [C][Fm]
   int* col_status;                     // [C]
+  int* col_nmu;                        // [C] NUMMU the column is solved with, 0: refused (k_atmo)
   // quadrature tables
   const double* gq_w;                  // Gauss-Legendre weights, packed: nquad=q at offset q*(q-1)/2
   int gq_max;
