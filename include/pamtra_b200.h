@@ -133,7 +133,8 @@ typedef struct pamtra_b200_columns {
   int32_t max_present;        /* upper bound on hydrometeor-bearing layers in the batch, 0 = ncol*max_nlyrs */
   int32_t nummu_mask;         /* bit 0: N=8, bit 1: N=16, bit 2: N=32 present; 0 = settings.nummu only */
   const pamtra_b200_species* species;  /* HOST pointer, [ncol or 1][nhydro] (copied by the library) */
-  const int32_t* nlyrs;       /* [ncol] */
+  const int32_t* nlyrs;       /* [ncol], 2 .. max_nlyrs; a column with another count is solved by no
+                                 kernel and gets PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE in status */
   const int32_t* nummu;       /* [ncol] in {8,16,32}; NULL = settings.nummu.  A column whose value is
                                  not 8/16/32, not in nummu_mask or above max_nummu is solved by no
                                  kernel and gets PAMTRA_B200_FATAL | PAMTRA_B200_ST_SIZE in status */
