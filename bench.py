@@ -303,7 +303,6 @@ def fp64_peak_tflops(dev):
 
 # k_layer<16> DRAM traffic per (layer, frequency) item: ncu capture of the
 # 256-column run (21,504 items): 13.7 MB read + 308.1 MB written per launch
-# (profiles/k_layer_fp64_dmma.md)
 LAYER_TRAFFIC_PER_ITEM = (13.749504e6 + 308.110848e6) / 21504
 
 
